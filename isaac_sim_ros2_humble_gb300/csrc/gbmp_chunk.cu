@@ -6,9 +6,10 @@
 
 namespace gbmp {
 
-// Warps per block of the chunk kernel.  Two blocks of 8 warps per SM at 128 registers
-// per thread: measured faster than 2 x 10 warps at 96 registers or 3 x 8 warps at 80,
-// where the chunk routine spills.
+// Warps per block of the chunk kernel: three blocks of 8 warps per SM at 80 registers.
+// The kernel is bound by instruction issue (0.72 of the issue slots at 65,536 edges), so
+// more warps bring little: 2.46 ms with two blocks, 2.22 ms with three, 2.21 ms with two
+// blocks of 16 warps at 64 registers (65,536 edges of the 8-DOF arm, verdicts).
 constexpr int kChunkWarps = 8;
 
 // Edge validation by chunks: a warp takes the next edge of `order` (a shared counter; the
@@ -23,9 +24,14 @@ constexpr int kChunkWarps = 8;
 // (uniform endpoints, 82 % colliding) the coarse-to-fine order checks 4.94 M states
 // against 8.89 M, 4.19 M of them on the free edges; 8 passes give 4.97 M (5.01 M in plain
 // order), 4 passes 5.06 M, a full bit-reversed order of the chunks 4.96 M.
+//
+// The chunk's states are tested side by side in the lanes (gbmp_chunk_device.cuh).
+// 65,536 edges, verdicts: 2.22 ms; 3.79 ms when the states were walked one by one, their
+// spheres in the lanes; 64 edges: 0.47 against 0.83 ms; 3,001 edges of a 30-link robot
+// with first hits: 1.20 against 1.73 ms.
 
-template <int SPL, int K, bool CNT>
-__global__ void __launch_bounds__(kChunkWarps *kWarp, 2)
+template <int K, bool CNT>
+__global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     k_edge_chunk(DevRobot R, DevEnv E, const float *__restrict__ from, const float *__restrict__ to,
                  const int *__restrict__ nsteps, const float *__restrict__ dir, const int *__restrict__ order,
                  long long n_edges, int *__restrict__ next, unsigned char *__restrict__ ok_out,
@@ -35,9 +41,8 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp, 2)
     SmemTables t = carve_tables(smem, R, nwords);
     if (!stage_tables(R, E, t, nwords)) return;
     const int warp = threadIdx.x / kWarp;
-    WarpScratch w;
     ChunkScratch cs;
-    carve_chunk(smem + smem_tables_bytes(R, nwords), R, K, warp, cs, w);
+    carve_chunk(smem + smem_tables_bytes(R, nwords), R, K, warp, cs);
     const int lane = threadIdx.x & 31;
     const bool any = first_hit_out == nullptr;
     for (;;) {
@@ -55,9 +60,8 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp, 2)
             const int nch = edge_chunk_count(n, K, any);
             for (int c = 0; c < nch; ++c) {
                 const StateRange r = edge_chunk_range(c, n, K, any);
-                const int h = warp_edge_chunk<SPL, K, CNT>(t, R, E, w, cs, lane, from + off, to + off, dir + off, r.x,
-                                                           r.y, n);
-                __syncwarp();
+                const int h = warp_edge_chunk<K, CNT>(t, R, E, cs, lane, from + off, to + off, dir + off, r.x, r.y, n,
+                                                      any);
                 if (h >= 0) { hit = h; break; }
             }
         }
@@ -69,34 +73,11 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp, 2)
     }
 }
 
-#define GBMP_CHUNK_SWITCH(spl, K, ...)                                                       \
-    do {                                                                                     \
-        if ((K) == 10) {                                                                     \
-            constexpr int KK = 10;                                                            \
-            switch (spl) {                                                                   \
-            case 1: { constexpr int SPL = 1; __VA_ARGS__; } break;                           \
-            case 2: { constexpr int SPL = 2; __VA_ARGS__; } break;                           \
-            case 3: { constexpr int SPL = 3; __VA_ARGS__; } break;                           \
-            case 4: { constexpr int SPL = 4; __VA_ARGS__; } break;                           \
-            case 5: { constexpr int SPL = 5; __VA_ARGS__; } break;                           \
-            case 6: { constexpr int SPL = 6; __VA_ARGS__; } break;                           \
-            case 7: { constexpr int SPL = 7; __VA_ARGS__; } break;                           \
-            default: { constexpr int SPL = 8; __VA_ARGS__; } break;                          \
-            }                                                                                \
-        } else {                                                                             \
-            constexpr int KK = 4;                                                            \
-            switch (spl) {                                                                   \
-            case 1: { constexpr int SPL = 1; __VA_ARGS__; } break;                           \
-            case 2: { constexpr int SPL = 2; __VA_ARGS__; } break;                           \
-            case 3: { constexpr int SPL = 3; __VA_ARGS__; } break;                           \
-            case 4: { constexpr int SPL = 4; __VA_ARGS__; } break;                           \
-            case 5: { constexpr int SPL = 5; __VA_ARGS__; } break;                           \
-            case 6: { constexpr int SPL = 6; __VA_ARGS__; } break;                           \
-            case 7: { constexpr int SPL = 7; __VA_ARGS__; } break;                           \
-            default: { constexpr int SPL = 8; __VA_ARGS__; } break;                          \
-            }                                                                                \
-        }                                                                                    \
-    } while (0)
+// The chunk kernel of K states a chunk (10 or 4), with or without work counting.
+static const void *edge_chunk_kernel(int K, bool count) {
+    if (K == 10) return count ? (const void *)k_edge_chunk<10, true> : (const void *)k_edge_chunk<10, false>;
+    return count ? (const void *)k_edge_chunk<4, true> : (const void *)k_edge_chunk<4, false>;
+}
 
 // States per chunk: 10 (three pose-row lanes per state fill 30 of 32 lanes in the chunk
 // FK; measured 8.22 ms against 8.43 for 8 on the 65,536-edge benchmark call), 4 for
@@ -109,20 +90,17 @@ int edge_chunk_states(const DevRobot &R, int form) {
 
 gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, int K, size_t *smem, int *grid) {
     *smem = smem_tables_bytes(R, env_words(E.ns, E.nb, E.nc)) + smem_chunk_bytes(R, K) * kChunkWarps;
-    gbmp_status st = GBMP_OK;
-    GBMP_CHUNK_SWITCH(R.spl, K, {
-        const void *fn = R.work ? (const void *)k_edge_chunk<SPL, KK, true> : (const void *)k_edge_chunk<SPL, KK, false>;
-        st = ensure_smem_optin(fn);
-        if (st) return st;
-        int per_sm = 0;
-        GBMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kChunkWarps * kWarp, *smem));
-        if (per_sm < 1) {
-            set_error("chunked edge kernel does not fit on an SM (%zu bytes of shared memory)", *smem);
-            st = GBMP_ERR_CAPACITY;
-        }
-        *grid = per_sm * num_sms;
-    });
-    return st;
+    const void *fn = edge_chunk_kernel(K, R.work != nullptr);
+    const gbmp_status st = ensure_smem_optin(fn);
+    if (st) return st;
+    int per_sm = 0;
+    GBMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kChunkWarps * kWarp, *smem));
+    if (per_sm < 1) {
+        set_error("chunked edge kernel does not fit on an SM (%zu bytes of shared memory)", *smem);
+        return GBMP_ERR_CAPACITY;
+    }
+    *grid = per_sm * num_sms;
+    return GBMP_OK;
 }
 
 gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int grid, size_t smem, cudaStream_t s,
@@ -131,14 +109,11 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
     // the grid is the resident blocks, at most one warp per edge
     const long long need = (n_edges + kChunkWarps - 1) / kChunkWarps;
     if (need < grid) grid = (int)need;
-    GBMP_CHUNK_SWITCH(R.spl, K, {
-        if (R.work)
-            k_edge_chunk<SPL, KK, true><<<grid, kChunkWarps * kWarp, smem, s>>>(R, E, from, to, nsteps, dir, order,
-                                                                                n_edges, next, ok, first_hit);
-        else
-            k_edge_chunk<SPL, KK, false><<<grid, kChunkWarps * kWarp, smem, s>>>(R, E, from, to, nsteps, dir, order,
-                                                                                 n_edges, next, ok, first_hit);
-    });
+    DevRobot r = R;
+    DevEnv e = E;
+    void *args[] = {&r, &e, &from, &to, &nsteps, &dir, &order, &n_edges, &next, &ok, &first_hit};
+    GBMP_CUDA(cudaLaunchKernel(edge_chunk_kernel(K, R.work != nullptr), dim3(grid), dim3(kChunkWarps * kWarp), args, smem,
+                               s));
     GBMP_CUDA(cudaGetLastError());
     return GBMP_OK;
 }
@@ -154,7 +129,7 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
 constexpr int kFkChunk = 10;
 
 __host__ __device__ inline size_t smem_fk_chunk_warp(const DevRobot &R) {
-    return 2 * align16(sizeof(float) * 12 * R.L * kFkChunk);
+    return align16(sizeof(float) * 12 * R.L * kFkChunk);
 }
 
 __global__ void __launch_bounds__(kChunkWarps *kWarp)
@@ -167,7 +142,6 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
     unsigned char *wbase = smem + smem_tables_bytes(R, 0) + smem_fk_chunk_warp(R) * warp;
     float *lpK = reinterpret_cast<float *>(wbase);
-    float *locK = reinterpret_cast<float *>(wbase + align16(sizeof(float) * 12 * R.L * kFkChunk));
     const int L = R.L, S = R.S;
     const long long nchunks = (n + kFkChunk - 1) / kFkChunk;
     const long long nw = (long long)gridDim.x * kChunkWarps;
@@ -175,7 +149,7 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
         const long long s0 = c * kFkChunk;
         const int ks = (int)min((long long)kFkChunk, n - s0);
         const float *qc = q + s0 * L;
-        warp_fk_chunk_q<kFkChunk>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, locK, lpK, lane);
+        warp_fk_chunk_q<kFkChunk>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, lpK, lane);
         if (poses) {
             if (vec) {
                 float4 *P4 = reinterpret_cast<float4 *>(poses + s0 * L * 16);

@@ -158,7 +158,7 @@ __device__ inline int block_nearest(const float *__restrict__ nodes, int size, i
 // chunks).  Returns true if every state is collision-free.
 template <int SPL, bool CULL, bool CHUNK>
 __device__ bool block_edge_free(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
-                                const WarpScratch &wc, const ChunkScratch &cs, const float *a, const float *b,
+                                const ChunkScratch &cs, const float *a, const float *b,
                                 float res, int rule, bool old_first, int *s_flag, float *s_dir, int *s_n) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x / kWarp;
     if (threadIdx.x == 0) {
@@ -196,7 +196,7 @@ __device__ bool block_edge_free(const SmemTables &t, const DevRobot &R, const De
             const int s0 = c0 + warp * per, s1 = min(s0 + per, last);
             int h = -1;
             if (s0 < s1)
-                h = warp_edge_chunk<SPL, kRrtcChunk, false>(t, R, E, wc, cs, lane, a, b, s_dir, s0, s1, nstates);
+                h = warp_edge_chunk<kRrtcChunk, false>(t, R, E, cs, lane, a, b, s_dir, s0, s1, nstates, true);
             if (h >= 0 && lane == 0) *s_flag = 1;
             __syncthreads();
             const bool any = *s_flag != 0;
@@ -295,8 +295,7 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
     int *s_misc = s_i + kRrtcWarps;                      // [8]
     unsigned char *act = reinterpret_cast<unsigned char *>(s_misc + 8);
     ChunkScratch cs{};
-    WarpScratch wc{};
-    if (CULL && CHUNK) carve_chunk(p + rrtc_misc_bytes(), R, kRrtcChunk, threadIdx.x / kWarp, cs, wc);
+    if (CULL && CHUNK) carve_chunk(p + rrtc_misc_bytes(), R, kRrtcChunk, threadIdx.x / kWarp, cs);
     for (int j = threadIdx.x; j < R.L; j += blockDim.x) act[j] = R.active[j];
     __syncthreads();
 
@@ -361,7 +360,7 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
             if (act[j] && scale < 1.f) q_s[j] = __fmaf_rn(scale, __fadd_rn(q_s[j], -q_a[j]), q_a[j]);
         __syncthreads();
         // 5. validate nn -> new, in path order (start tree: nn first; goal tree: new first)
-        if (!block_edge_free<SPL, CULL, CHUNK>(t, R, E, w, wc, cs, tr == 0 ? q_a : q_s, tr == 0 ? q_s : q_a, prm.res, prm.rule,
+        if (!block_edge_free<SPL, CULL, CHUNK>(t, R, E, w, cs, tr == 0 ? q_a : q_s, tr == 0 ? q_s : q_a, prm.res, prm.rule,
                                         tr == 0, s_misc + 4, s_dir, s_misc + 5)) {
             if (prm.dd && threadIdx.x == 0) dd_update(P.radii[tr] + nn, true, prm);
             continue;
@@ -402,7 +401,7 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
             __syncthreads();
             // in path order: the last step joins the goal tree's node to the start tree's
             // (start tree first), every other step runs away from its tree's root
-            if (!block_edge_free<SPL, CULL, CHUNK>(t, R, E, w, wc, cs, tr == 0 ? q_a : q_c, tr == 0 ? q_c : q_a, prm.res, prm.rule,
+            if (!block_edge_free<SPL, CULL, CHUNK>(t, R, E, w, cs, tr == 0 ? q_a : q_c, tr == 0 ? q_c : q_a, prm.res, prm.rule,
                                             tr == 0, s_misc + 4, s_dir, s_misc + 5)) {
                 connected = false;
                 break;

@@ -1,0 +1,74 @@
+"""The chunk kernel of edge validation (states of a chunk side by side in the lanes)
+against the state-by-state kernel: identical verdicts and first hits, where the chunk's
+items do not fill the lanes evenly or do not take the common path."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from isaac_sim_ros2_humble_gb300 import api, workloads as W
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _run(R, E, a, b, res, first_hit):
+    n = a.shape[0]
+    ok = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+    fh = torch.full((n,), 99, dtype=torch.int32, device="cuda")
+    api.check_edges(R, E, a, b, res, 1, ok, fh if first_hit else None)
+    torch.cuda.synchronize()
+    return ok.cpu().numpy(), fh.cpu().numpy()
+
+
+def _forms_agree(robot, env, n, res, forms=(4, 10), seed=5):
+    R, E = api.Robot(robot), api.Env(env)
+    rng = np.random.default_rng(seed)
+    a, b = (torch.from_numpy(robot.sample_full(rng, n)).cuda() for _ in range(2))
+    R.set_edge_form(1)
+    ok, fh = _run(R, E, a, b, res, True)
+    np.testing.assert_array_equal(ok, fh == -1)
+    for form in forms:
+        R.set_edge_form(form)
+        ok_f, fh_f = _run(R, E, a, b, res, True)
+        np.testing.assert_array_equal(fh_f, fh)
+        np.testing.assert_array_equal(ok_f, ok)
+        np.testing.assert_array_equal(_run(R, E, a, b, res, False)[0], ok)
+    return ok
+
+
+@pytest.mark.parametrize("n_spheres", [1, 7, 33, 57, 200])
+def test_odd_sphere_counts(n_spheres):
+    robot = W.serial_arm(51, dof=7, n_spheres=n_spheres, radius_range=(0.02, 0.05))
+    ok = _forms_agree(robot, W.random_env(52, 33, 5, 3, oriented=True), 513, 0.03)
+    assert 0 < ok.sum() < len(ok)
+
+
+def test_one_sided_link_mask_takes_the_pair_list():
+    """A mask that enables (link of the lower sphere index, link of the higher) one way
+    only, with the spheres in random order: the pairs of two groups are then not all
+    (sphere of a, sphere of b) pairs, and the pair list decides."""
+    base = W.serial_arm(53, dof=6, n_spheres=60, radius_range=(0.03, 0.06))
+    order = np.random.default_rng(3).permutation(60)
+    robot = dataclasses.replace(base, sphere_link=base.sphere_link[order], sphere_pos=base.sphere_pos[order],
+                                sphere_r=base.sphere_r[order], enables=np.triu(base.enables, 1).astype(np.uint8))
+    ok = _forms_agree(robot, W.Environment.empty(), 600, 0.03)
+    assert 0 < ok.sum() < len(ok)
+
+
+def test_branching_robot_with_many_links():
+    """A robot of 20 links (4 states a chunk): parents that are not the previous link."""
+    t = W.tree_robot(4, n_spheres=60)
+    parent = np.concatenate([t.parent, [9, 10, 8, 12, 2, 14, 14, 5, 17, 1]]).astype(np.int32)
+    L = len(parent)
+    ext = lambda a, fill: np.concatenate([a, np.full((L - len(t.parent),) + a.shape[1:], fill, a.dtype)])   # noqa: E731
+    poses = ext(t.joint_poses, 0)
+    poses[len(t.parent):] = t.joint_poses[1]
+    enables = np.zeros((L, L), np.uint8)
+    enables[: len(t.parent), : len(t.parent)] = t.enables
+    robot = dataclasses.replace(t, parent=parent, joint_types=ext(t.joint_types, W.REVOLUTE), joint_poses=poses,
+                                joint_axes=ext(t.joint_axes, 1.0), active=ext(t.active, 1),
+                                lower=ext(t.lower, -2.0), upper=ext(t.upper, 2.0), default=ext(t.default, 0.0),
+                                enables=enables, link_names=["l%d" % i for i in range(L)])
+    ok = _forms_agree(robot, W.random_env(54, 40, 8, 4, oriented=True), 400, 0.03, forms=(0, 4, 10))
+    assert 0 < ok.sum() < len(ok)
