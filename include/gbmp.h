@@ -222,8 +222,8 @@ GBMP_API gbmp_status gbmp_check_batch_destroy(gbmp_check_batch batch);
  * resolution.  Asynchronous: three launches on `stream`, no host synchronisation (the
  * reference reads step counts back to the host, SingleArmSpace.cu:728-739).  The working
  * memory belongs to the robot handle: calls with one robot on different streams must be
- * ordered by the caller.  Each edge is validated by one warp, stopping at a colliding
- * state; the edges are taken longest first.  Robots of up to 32 sphere-carrying links are
+ * ordered by the caller.  The edges are taken longest first, each cut into parts
+ * that different warps validate, stopping at a colliding state.  Robots of up to 32 sphere-carrying links are
  * validated by chunks of consecutive states (10 states; 4 for robots of more than 16
  * links), others state by state; gbmp_robot_set_edge_form overrides the form for one
  * robot handle.  With d_first_hit the chunks go in state order (the first 4 states, then

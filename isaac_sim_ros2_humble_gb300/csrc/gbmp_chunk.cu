@@ -12,12 +12,20 @@ namespace gbmp {
 // blocks of 16 warps at 64 registers (65,536 edges of the 8-DOF arm, verdicts).
 constexpr int kChunkWarps = 8;
 
-// Edge validation by chunks: a warp takes the next edge of `order` (a shared counter; the
-// edges come longest first, so the last edges taken are the shortest and the warps end
-// together), walks its states in chunks of consecutive states and stops at the first chunk
-// that holds a colliding state.  One warp per edge, so no state past that hit is placed in
-// a later chunk.  Writes the edge's outputs (ok, first hit; -2 for an edge too long to
-// validate).
+// Edge validation by chunks.  An edge's chunks, in their order, are cut into parts of
+// consecutive chunks (EdgePlan, made by k_edge_order from the lengths); item i is part
+// i / n_edges of edge order[i % n_edges], so part 0 of every edge comes first, the edges of
+// each part longest first.  A warp takes `grab` items from a shared counter, drops those
+// that are settled already (past the edge's end, or another part has recorded a hit that
+// decides), one lane each, and walks the chunks of the others up to a chunk that holds a
+// colliding state.  k_edge_order has written the outputs of a free edge (and of one too
+// long to validate, which no warp walks); a hit clears ok and lowers the first hit (-1,
+// the largest unsigned value, until then).
+//
+// Why parts: the free edges are few (18 % of the benchmark's) and long, so with one warp
+// per edge most warps idled while some walked up to 56 chunks in a row: 64 edges 0.47 ms
+// whole, 0.046 ms in parts; 3,001 edges of a 30-link robot with first hits 1.20 and 0.30
+// ms; 65,536 edges (18 for each warp) 2.22 and 2.26 ms.
 //
 // The chunk orders are gbmp_order.h's: state order when the first hit is asked for,
 // coarse to fine when only the verdict is.  On the 65,536 edges of the 8-DOF benchmark
@@ -27,15 +35,14 @@ constexpr int kChunkWarps = 8;
 //
 // The chunk's states are tested side by side in the lanes (gbmp_chunk_device.cuh).
 // 65,536 edges, verdicts: 2.22 ms; 3.79 ms when the states were walked one by one, their
-// spheres in the lanes; 64 edges: 0.47 against 0.83 ms; 3,001 edges of a 30-link robot
-// with first hits: 1.20 against 1.73 ms.
+// spheres in the lanes.
 
 template <int K, bool CNT>
 __global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     k_edge_chunk(DevRobot R, DevEnv E, const float *__restrict__ from, const float *__restrict__ to,
                  const int *__restrict__ nsteps, const float *__restrict__ dir, const int *__restrict__ order,
-                 long long n_edges, int *__restrict__ next, unsigned char *__restrict__ ok_out,
-                 int *__restrict__ first_hit_out) {
+                 int n_edges, const EdgePlan *__restrict__ plan, unsigned long long *__restrict__ next,
+                 unsigned char *ok_out, int *first_hit_out) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nwords = env_words(E.ns, E.nb, E.nc);
     SmemTables t = carve_tables(smem, R, nwords);
@@ -45,29 +52,50 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     carve_chunk(smem + smem_tables_bytes(R, nwords), R, K, warp, cs);
     const int lane = threadIdx.x & 31;
     const bool any = first_hit_out == nullptr;
+    const int parts = plan->parts, span0 = plan->span, grab = plan->grab;
+    const long long items = (long long)n_edges * parts;
+    // the other warps' findings (relaxed reads: a late look costs a chunk, not the result)
+    auto settled = [&](int e, int first_state) {
+        return any ? ok_out && *(volatile unsigned char *)(ok_out + e) == 0
+                   : *(volatile unsigned *)(first_hit_out + e) <= (unsigned)first_state;
+    };
     for (;;) {
-        int i = 0;
-        if (lane == 0) i = atomicAdd(next, 1);
-        i = __shfl_sync(kFull, i, 0);
-        if (i >= n_edges) break;
-        const int e = order[i];
-        const int n = nsteps[e];
-        int hit = -1;
-        if (n > kMaxEdgeStates) {
-            hit = -2;   // too long to validate
-        } else {
-            const long long off = (long long)e * R.L;
-            const int nch = edge_chunk_count(n, K, any);
-            for (int c = 0; c < nch; ++c) {
-                const StateRange r = edge_chunk_range(c, n, K, any);
-                const int h = warp_edge_chunk<K, CNT>(t, R, E, cs, lane, from + off, to + off, dir + off, r.x, r.y, n,
-                                                      any);
-                if (h >= 0) { hit = h; break; }
+        unsigned long long i0 = 0;
+        if (lane == 0) i0 = atomicAdd(next, (unsigned long long)grab);
+        i0 = __shfl_sync(kFull, i0, 0);
+        if ((long long)i0 >= items) break;
+        const long long i = (long long)i0 + lane;
+        int e = 0, n = 0, c0 = 0, c1 = 0;
+        if (lane < grab && i < items) {
+            const int p = (int)(i / n_edges);
+            e = order[i - (long long)p * n_edges];
+            n = nsteps[e];
+            if (n <= kMaxEdgeStates) {
+                const int nch = edge_chunk_count(n, K, any);
+                const int span = max(span0, (nch + parts - 1) / parts);
+                c0 = p * span;
+                c1 = min(c0 + span, nch);
+                if (p > 0 && c0 < c1 && settled(e, edge_chunk_range(c0, n, K, any).x)) c1 = c0;
             }
         }
-        if (lane == 0) {
-            if (ok_out) ok_out[e] = hit == -1;
-            if (first_hit_out) first_hit_out[e] = hit;
+        for (unsigned live = __ballot_sync(kFull, c0 < c1); live; live &= live - 1u) {
+            const int x = __ffs(live) - 1;
+            const int we = __shfl_sync(kFull, e, x), wn = __shfl_sync(kFull, n, x);
+            const int wc0 = __shfl_sync(kFull, c0, x), wc1 = __shfl_sync(kFull, c1, x);
+            const long long off = (long long)we * R.L;
+            for (int c = wc0; c < wc1; ++c) {
+                const StateRange r = edge_chunk_range(c, wn, K, any);
+                if (parts > 1 && c > wc0 && __any_sync(kFull, settled(we, r.x))) break;
+                const int h = warp_edge_chunk<K, CNT>(t, R, E, cs, lane, from + off, to + off, dir + off, r.x, r.y, wn,
+                                                      any);
+                if (h >= 0) {
+                    if (lane == 0) {
+                        if (ok_out) *(volatile unsigned char *)(ok_out + we) = 0;
+                        if (first_hit_out) atomicMin(reinterpret_cast<unsigned *>(first_hit_out + we), (unsigned)h);
+                    }
+                    break;
+                }
+            }
         }
         __syncwarp();
     }
@@ -103,15 +131,19 @@ gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, 
     return GBMP_OK;
 }
 
+int edge_chunk_warps(int grid) { return grid * kChunkWarps; }
+
 gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int grid, size_t smem, cudaStream_t s,
                               const float *from, const float *to, const int *nsteps, const float *dir,
-                              const int *order, long long n_edges, int *next, unsigned char *ok, int *first_hit) {
-    // the grid is the resident blocks, at most one warp per edge
-    const long long need = (n_edges + kChunkWarps - 1) / kChunkWarps;
+                              const int *order, long long n_edges, const EdgePlan *plan, unsigned long long *next,
+                              unsigned char *ok, int *first_hit) {
+    // the grid is the resident blocks, at most one warp per item
+    const long long need = (n_edges * kEdgeMaxParts + kChunkWarps - 1) / kChunkWarps;
     if (need < grid) grid = (int)need;
+    int ne = (int)n_edges;
     DevRobot r = R;
     DevEnv e = E;
-    void *args[] = {&r, &e, &from, &to, &nsteps, &dir, &order, &n_edges, &next, &ok, &first_hit};
+    void *args[] = {&r, &e, &from, &to, &nsteps, &dir, &order, &ne, &plan, &next, &ok, &first_hit};
     GBMP_CUDA(cudaLaunchKernel(edge_chunk_kernel(K, R.work != nullptr), dim3(grid), dim3(kChunkWarps * kWarp), args, smem,
                                s));
     GBMP_CUDA(cudaGetLastError());

@@ -141,17 +141,53 @@ __global__ void k_edge_setup(const float *__restrict__ from, const float *__rest
 
 // Processing order of the edges, longest bucket first: order[slot] = edge, the slots of a
 // bucket following the counts of the longer buckets (hist) in arrival order (cursor).
+// Also writes the outputs of an edge without a collision, which validation then changes
+// where it finds one: ok 1, first hit -1 (an edge too long to validate: ok 0, -2).
+// With K > 0 (validation by chunks of K states on `warps` warps) it also makes the plan
+// that cuts the edges into items: parts of `span` chunks so that a quarter of all chunks
+// (what is left of them when the colliding edges stop early) gives each warp about
+// kItemsPerWarp items, up to kEdgeMaxParts parts for the longest edge, and `grab` items a time
+// so that each warp comes back about kGrabsPerWarp times (65,536 edges: 2.26 ms with 32,
+// 2.32 with 16, 2.45 with 8; 17,339 shorter edges 0.312, 0.318 and 0.373 ms; 4 or 16 items
+// a warp instead of 8 cost up to 10 % on batches of 17,000 to 33,000 edges).
+constexpr int kItemsPerWarp = 8, kGrabsPerWarp = 32, kMaxSpan = 8;
 __global__ void k_edge_order(const int *__restrict__ nsteps, long long E, const int *__restrict__ hist,
-                             int *__restrict__ cursor, int *__restrict__ order) {
+                             int *__restrict__ cursor, int *__restrict__ order, unsigned char *__restrict__ ok,
+                             int *__restrict__ first_hit, int K, int warps, EdgePlan *__restrict__ plan) {
     __shared__ int base[kEdgeBuckets];
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int b = 0; b < kEdgeBuckets; ++b) { base[b] = acc; acc += hist[b]; }
+    static_assert(kEdgeBuckets == 2 * kWarp, "two buckets a lane");
+    if (threadIdx.x < kWarp) {
+        const int lane = threadIdx.x, b0 = 2 * lane;
+        const int h0 = hist[b0], h1 = hist[b0 + 1];
+        int acc = h0 + h1;   // edges up to this lane's buckets
+        for (int off = 1; off < kWarp; off <<= 1) {
+            const int v = __shfl_up_sync(kFull, acc, off);
+            if (lane >= off) acc += v;
+        }
+        base[b0] = acc - h1 - h0;
+        base[b0 + 1] = acc - h1;
+        if (K && blockIdx.x == 0) {
+            // chunks of an edge of bucket b: about (16 (63 - b) + 8) / K
+            float chunks = (float)h0 * (1 + (16 * (kEdgeBuckets - 1 - b0) + 8) / K) +
+                           (float)h1 * (1 + (16 * (kEdgeBuckets - 2 - b0) + 8) / K);
+            for (int off = 16; off; off >>= 1) chunks += __shfl_xor_sync(kFull, chunks, off);
+            const int first = __ffs(__ballot_sync(kFull, h0 + h1 > 0)) - 1;   // E > 0: some bucket holds an edge
+            const int longest = 2 * first + (__shfl_sync(kFull, h0, first) ? 0 : 1);
+            if (lane == 0) {
+                const int most = 2 + 16 * (kEdgeBuckets - longest) / K;   // chunks of the longest edge (longer: bucket 0)
+                const int span = max(1, min(kMaxSpan, (int)(chunks / (4.f * kItemsPerWarp * warps))));
+                const int parts = max(1, min(kEdgeMaxParts, (most + span - 1) / span));
+                const int grab = (int)max(1LL, min(32LL, E * parts / ((long long)kGrabsPerWarp * warps)));
+                *plan = EdgePlan{parts, span, grab, 0};
+            }
+        }
     }
     __syncthreads();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < E; k += (long long)gridDim.x * blockDim.x) {
-        const int b = edge_bucket(nsteps[k]);
+        const int n = nsteps[k], b = edge_bucket(n);
         order[base[b] + atomicAdd(cursor + b, 1)] = (int)k;
+        if (ok) ok[k] = n <= kMaxEdgeStates;
+        if (first_hit) first_hit[k] = n <= kMaxEdgeStates ? -1 : -2;
     }
 }
 
@@ -822,15 +858,16 @@ gbmp_status gbmp_robot_set_edge_form(gbmp_robot r, int32_t form) {
 // gbmp_check_edges_noalloc uses one fixed array that the library holds on each device.
 // Three launches, no host round trip:
 //   k_edge_setup   step count, direction and length per edge, length histogram;
-//   k_edge_order   the edges in longest-first order (counting sort by buckets);
-//   validation     a warp takes the next edge of that order (shared counter), walks its
-//                  states in order (chunks of consecutive states, or state by state) and
-//                  stops at the first colliding state; it writes the edge's outputs.
+//   k_edge_order   the edges in longest-first order (counting sort by buckets), the
+//                  outputs of edges without a collision, and the plan of parts;
+//   validation     warps take parts of edges in that order (chunks of consecutive
+//                  states), or whole edges (state by state), from a shared counter and
+//                  stop at a colliding state, which changes the edge's outputs.
 // Working memory of E edges of L links:
 //   nsteps[E], order[E]   int
 //   dir[E*L]              float
-//   ctr[kEdgeCtrInts]     int    MUST START AT ZERO (hist[64], cursor[64], next):
-//                                zeroed on the stream by every call
+//   ctr[kEdgeCtrInts]     int    MUST START AT ZERO (hist[64], cursor[64], next; then
+//                                the EdgePlan): zeroed on the stream by every call
 // ---------------------------------------------------------------------------------
 namespace gbmp {
 
@@ -860,6 +897,7 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
                                  int32_t *d_num_steps, cudaStream_t s, const EdgeScratch &sc) {
     int *nsteps = sc.nsteps, *order = sc.order, *ctr = sc.ctr;
     int *hist = ctr, *cursor = ctr + kEdgeBuckets, *next = ctr + 2 * kEdgeBuckets;
+    EdgePlan *plan = reinterpret_cast<EdgePlan *>(next + 4);   // next: 8 bytes, 16-byte aligned
     float *dir = sc.dir;
     const int L = r->L;
     GBMP_CUDA(cudaMemsetAsync(ctr, 0, kEdgeCtrInts * sizeof(int), s));
@@ -874,13 +912,6 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
         k_edge_setup<<<blocks, tb, 0, s>>>(d_from, d_to, E, L, res, rule, nsteps, dir, hist, d_length, d_num_steps);
     }
     GBMP_CUDA(cudaGetLastError());
-    {
-        ProfScope ps(GBMP_PROF_OTHER, s);
-        k_edge_order<<<(unsigned)std::min<long long>(blocks, 4LL * r->num_sms), tb, 0, s>>>(nsteps, E, hist, cursor,
-                                                                                            order);
-    }
-    GBMP_CUDA(cudaGetLastError());
-
     const DevEnv Ev = env->dev();
     DevRobot D = r->dev;
     D.work = work_counter();
@@ -906,13 +937,21 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
         });
     }
     if (st) return st;
-    const long long need = (E + kWarpsPerBlock - 1) / kWarpsPerBlock;   // one warp per edge at most
-    if (need < grid) grid = (int)need;
+    {
+        ProfScope ps(GBMP_PROF_OTHER, s);
+        k_edge_order<<<(unsigned)std::min<long long>(blocks, 4LL * r->num_sms), tb, 0, s>>>(
+            nsteps, E, hist, cursor, order, d_ok, d_first_hit, K, edge_chunk_warps(grid), plan);
+    }
+    GBMP_CUDA(cudaGetLastError());
+    if (!K) {   // one warp per edge at most
+        const long long need = (E + kWarpsPerBlock - 1) / kWarpsPerBlock;
+        if (need < grid) grid = (int)need;
+    }
     {
         ProfScope ps(GBMP_PROF_EDGE_WAVE, s);
         if (K) {
-            st = edge_chunk_launch(Dc, Ev, K, grid, smem, s, d_from, d_to, nsteps, dir, order, E, next, d_ok,
-                                   d_first_hit);
+            st = edge_chunk_launch(Dc, Ev, K, grid, smem, s, d_from, d_to, nsteps, dir, order, E, plan,
+                                   reinterpret_cast<unsigned long long *>(next), d_ok, d_first_hit);
             if (st) return st;
         } else {
             GBMP_SPL_SWITCH(r->dev.spl, {

@@ -138,6 +138,14 @@ gbmp_status codegen_fk(const gbmp_robot_s *r, const float *q, long long n, float
 gbmp_status codegen_edge_setup(const gbmp_robot_s *r, const float *from, const float *to, long long E, float res,
                                int rule, int *nsteps, float *dir, int *hist, float *length_out, int *nsteps_out,
                                cudaStream_t s);
+// How a call's edges are cut into items (gbmp_chunk.cu): parts per edge, the least chunks
+// of a part, and the items a warp takes at a time.  Made on the device by k_edge_order.
+constexpr int kEdgeMaxParts = 64;
+struct EdgePlan {
+    int parts, span, grab, pad;
+};
+// Warps of the chunk kernel resident in `grid` blocks.
+int edge_chunk_warps(int grid);
 // Edge validation by chunks of consecutive states (gbmp_chunk.cu).  K = states per
 // chunk for this robot (0: use the per-state kernels); `form` is the robot handle's
 // edge_form (0 automatic, 1 per state, 4 or 10 states per chunk).
@@ -148,7 +156,8 @@ gbmp_status fk_chunk_launch(const DevRobot &R, int num_sms, const float *q, long
 gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, int K, size_t *smem, int *grid);
 gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int grid, size_t smem, cudaStream_t s,
                               const float *from, const float *to, const int *nsteps, const float *dir,
-                              const int *order, long long n_edges, int *next, unsigned char *ok, int *first_hit);
+                              const int *order, long long n_edges, const EdgePlan *plan, unsigned long long *next,
+                              unsigned char *ok, int *first_hit);
 }  // namespace gbmp
 
 struct gbmp_env_s {

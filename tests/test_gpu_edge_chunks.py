@@ -72,3 +72,29 @@ def test_branching_robot_with_many_links():
                                 enables=enables, link_names=["l%d" % i for i in range(L)])
     ok = _forms_agree(robot, W.random_env(54, 40, 8, 4, oriented=True), 400, 0.03, forms=(0, 4, 10))
     assert 0 < ok.sum() < len(ok)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 57, 300, 4000])
+@pytest.mark.parametrize("res", [0.004, 0.02, 3.0])
+def test_edges_cut_into_parts(n, res):
+    """From a single edge (all of its chunks at once on different warps) to more edges than
+    warps; long edges (up to 1,400 states, past the last length bucket), and edges of one
+    or two states."""
+    robot = W.serial_arm(55, dof=7, n_spheres=50)
+    ok = _forms_agree(robot, W.random_env(56, 24, 6, 2, oriented=True), n, res, forms=(0,), seed=n)
+    if n >= 300:
+        assert 0 < ok.sum() < n
+
+
+def test_outputs_of_long_and_free_edges_without_any_hit():
+    """Edges too long to validate beside free ones: the outputs that no warp touches."""
+    robot = W.serial_arm(57, dof=6, n_spheres=12, radius_range=(0.01, 0.02))
+    robot.enables[:] = 0
+    R, E = api.Robot(robot), api.Env(W.Environment.empty())
+    a = torch.zeros((5, robot.num_links), device="cuda")
+    b = a.clone()
+    b[1, 2], b[3, 1] = 2.0, 1e-3
+    ok, fh = _run(R, E, a, b, 2e-7, True)
+    np.testing.assert_array_equal(ok, [1, 0, 1, 1, 1])
+    np.testing.assert_array_equal(fh, [-1, -2, -1, -1, -1])
+    np.testing.assert_array_equal(_run(R, E, a, b, 2e-7, False)[0], ok)
