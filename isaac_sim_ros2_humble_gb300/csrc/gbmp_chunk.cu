@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
     k_fk_chunk(DevRobot R, const float *__restrict__ q, long long n, float *__restrict__ poses,
                float *__restrict__ centers, int vec) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const DevEnv E{0, 0, 0, nullptr};
+    const DevEnv E{};
     SmemTables t = carve_tables(smem, R, 0);
     if (!stage_tables(R, E, t, 0)) return;
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;

@@ -11,9 +11,10 @@
 //      piece of a link's spheres) over the chunk by an axis-aligned box;
 //   B. turns each box into a swept group sphere: centre = box centre, radius = half the
 //      box diagonal + the group radius (which already carries kBroadMargin);
-//   C. runs the broad phase ONCE for the chunk: the bounding sphere of every run of 32
-//      obstacles (scenes store obstacles in spatially compact runs) against the swept
-//      group spheres, then the obstacles of the runs some group touches against those
+//   C. runs the broad phase ONCE for the chunk: the swept group spheres that the scene's
+//      distance field does not clear (scene_far, one load a group, all groups at once)
+//      against the bounding sphere of every run of 32 obstacles (scenes store obstacles
+//      in spatially compact runs), then the obstacles of the runs some group touches against those
 //      groups; an obstacle that touches any is tested exactly at once (D);
 //   D. exact tests with the chunk's states side by side in the lanes: (state, sphere)
 //      against an obstacle, (state, group pair) for the self pairs, whose overlapping
@@ -25,7 +26,8 @@
 // equal the per-state kernel's.
 //
 // What bounds it: instruction issue and latency, not memory (the tables live in shared
-// memory).  Walking the states one after another left most lanes idle: per state of the
+// memory).  65,536 edges of the benchmark: 2.26 ms when every swept sphere was tested
+// against every run, 1.25 ms with the field (most chunks then have no group left).  Walking the states one after another left most lanes idle: per state of the
 // benchmark's edges 0.3 obstacle candidates and 2.3 group pairs, each pair's test a chain
 // of shared-memory loads over 7 spheres.  Side by side the chunk's 23 (state, pair) items
 // fill a warp.
@@ -122,15 +124,16 @@ __device__ inline void warp_fk_chunk(const SmemTables &t, int L, int ks, const f
         lpK, lane);
 }
 
-// Groups (bit q) whose swept sphere touches the bounding sphere of run c0 + lane of an
-// obstacle type with nruns runs; 0 for lanes past the last run.
-__device__ __forceinline__ unsigned run_groups(const float4 *runs, int nruns, int c0, const ChunkScratch &cs, int G,
-                                               int lane) {
+// Groups of `groups` (bit q) whose swept sphere touches the bounding sphere of run c0 +
+// lane of an obstacle type with nruns runs; 0 for lanes past the last run.
+__device__ __forceinline__ unsigned run_groups(const float4 *runs, int nruns, int c0, const ChunkScratch &cs,
+                                               unsigned groups, int lane) {
     const int c = c0 + lane;
     unsigned gm = 0u;
     if (c < nruns) {
         const float4 b = runs[c];
-        for (int q = 0; q < G; ++q) {
+        for (unsigned m = groups; m; m &= m - 1u) {
+            const int q = __ffs(m) - 1;
             const float4 gs = cs.sgb[q];
             const float rr = gs.w + b.w;
             if (sq3(gs.x - b.x, gs.y - b.y, gs.z - b.z) < rr * rr) gm |= 1u << q;
@@ -354,14 +357,18 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
         hiz = fmaxf(hiz, __shfl_xor_sync(kFull, hiz, off));
     }
 
-    // --- B: swept group spheres ---
+    // --- B: swept group spheres; those that the scene's distance field cannot clear ---
+    bool is_near = false;
     if (lane < R.G) {
         const float cx = 0.5f * (lox + hix), cy = 0.5f * (loy + hiy), cz = 0.5f * (loz + hiz);
         const float hx = 0.5f * (hix - lox), hy = 0.5f * (hiy - loy), hz = 0.5f * (hiz - loz);
         const float rad = sqrtf(hx * hx + hy * hy + hz * hz) + gr;
         cs.sgb[lane] = make_float4(cx, cy, cz, rad);
         cs.sgA[lane] = __fmaf_rn(cz, cz, __fmaf_rn(cy, cy, __fmaf_rn(cx, cx, -rad * rad)));
+        is_near = !scene_far(E, cx, cy, cz, rad);
     }
+    const unsigned near_groups = __ballot_sync(kFull, is_near);
+    if (CNT) fl += (unsigned long long)R.G * kFlField;
     __syncwarp();
 
     int kmax = ks;   // states below kmax are not yet known to collide (any: kmax == ks)
@@ -384,10 +391,10 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
     const float4 *runs_w = t.env + env_cluster_base(E.ns, E.nb, E.nc);
     bool done = false;
 #pragma unroll 1
-    for (int c0 = 0; c0 < nrun && !done; c0 += kWarp) {
-        const unsigned gmc = run_groups(runs_w, nrun, c0, cs, R.G, lane);
+    for (int c0 = 0; c0 < nrun && near_groups && !done; c0 += kWarp) {
+        const unsigned gmc = run_groups(runs_w, nrun, c0, cs, near_groups, lane);
         unsigned runs = __ballot_sync(kFull, gmc != 0u);
-        if (CNT) fl += (unsigned long long)min(kWarp, nrun - c0) * R.G * kFlGroupPair;
+        if (CNT) fl += (unsigned long long)min(kWarp, nrun - c0) * __popc(near_groups) * kFlGroupPair;
         while (runs && !done) {
             const int j = __ffs(runs) - 1;
             runs &= runs - 1u;

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     k_fk(DevRobot R, const float *__restrict__ q, long long n, float *__restrict__ poses,
          float *__restrict__ centers) {
     extern __shared__ __align__(16) unsigned char smem[];
-    DevEnv E{0, 0, 0, nullptr};
+    DevEnv E{};
     SmemTables t = carve_tables(smem, R, 0);
     if (!stage_tables(R, E, t, 0)) return;
     WarpScratch w = carve_warp(smem + smem_tables_bytes(R, 0), R, threadIdx.x / kWarp);
@@ -744,9 +744,26 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     cluster_spheres(sc, srd, os, runs);
     cluster_spheres(bc, brd, ob, runs + env_clusters(ns));
     cluster_spheres(cc, crd, oc, runs + env_clusters(ns) + env_clusters(nb));
-    cudaError_t err = cudaMalloc(&e->d_words, sizeof(float4) * e->h_words.size());
-    if (err == cudaSuccess)
-        err = cudaMemcpy(e->d_words, e->h_words.data(), sizeof(float4) * e->h_words.size(), cudaMemcpyHostToDevice);
+    DevEnv &E = e->view;
+    E.ns = ns; E.nb = nb; E.nc = nc;
+    std::vector<double> bounds;
+    auto bound = [&](const std::vector<double> &c, const std::vector<double> &r) {
+        for (size_t i = 0; i < r.size(); ++i) bounds.insert(bounds.end(), {c[3 * i], c[3 * i + 1], c[3 * i + 2], r[i]});
+    };
+    bound(sc, srd);
+    bound(bc, brd);
+    bound(cc, crd);
+    const bool field = scene_field_plan(bounds, E);
+    const size_t wbytes = sizeof(float4) * e->h_words.size();
+    cudaError_t err = cudaMalloc(&e->d_words, wbytes + (field ? sizeof(float) * (size_t)E.nx * E.ny * E.nz : 0));
+    if (err == cudaSuccess) err = cudaMemcpy(e->d_words, e->h_words.data(), wbytes, cudaMemcpyHostToDevice);
+    E.words = e->d_words;
+    if (err == cudaSuccess && field) {
+        float *values = reinterpret_cast<float *>(e->d_words + e->h_words.size());
+        err = scene_field_build(E, values, nullptr);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
+        E.field = values;
+    }
     if (err != cudaSuccess) {
         set_error("uploading environment failed: %s", cudaGetErrorString(err));
         gbmp_env_destroy(e);

@@ -98,7 +98,22 @@ constexpr float kBroadMargin = 1e-3f;    // metres added to every group bounding
 struct DevEnv {
     int ns, nb, nc;
     const float4 *words;              // env_words(ns, nb, nc) float4
+    // Distance field of the scene (gbmp_field.cu), or null: field[(iz * ny + iy) * nx + ix]
+    // is the least distance from the centre of cell (ix, iy, iz) to an obstacle; cells of
+    // edge h from the corner (ox, oy, oz); [lo, hi] bounds all obstacles.
+    const float *field;
+    int nx, ny, nz;
+    float ox, oy, oz, h, inv_h;
+    float lox, loy, loz, hix, hiy, hiz;
 };
+
+// Cells along the field's longest side (128 KB a scene at most).  65,536 edges of the 8-DOF
+// arm in 336 obstacles: 1.255 ms with 32, 1.242 with 48, 1.238 with 64, 1.233 with 128;
+// a scene of 336 obstacles takes 42 us longer to create (72 us; 60 us longer with 48).
+constexpr int kFieldCells = 32;
+constexpr double kFieldBorder = 0.2;     // metres of field around the obstacles
+constexpr double kFieldLargest = 1.0;    // bounding radius of the obstacles that span the field
+constexpr int kFlField = 24;             // box distance, cell and bound of one lookup
 
 __host__ __device__ inline int env_clusters(int n) { return (n + 31) / 32; }
 __host__ __device__ inline int env_cluster_base(int ns, int nb, int nc) { return 2 * ns + (ns + 3) / 4 + 5 * nb + 4 * nc; }
@@ -392,6 +407,26 @@ __device__ __forceinline__ float3 xform_rows(const float4 r0, const float4 r1, c
 
 __device__ __forceinline__ float sq3(float dx, float dy, float dz) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+// True when no obstacle of the scene comes within `rad` of (x, y, z): the sphere lies
+// outside the box of all obstacles, or the distance stored for the nearest cell centre,
+// less the way there (distances change by no more than the way), exceeds rad.  False says
+// nothing.  One load (L1 or L2: a field is 128 KB at most) in place of a test
+// against every obstacle; with the cells of a 2 m scene 6 cm wide the bound is 3 cm short on
+// average.
+// Callers' radii carry kBroadMargin, which covers the rounding here and in the exact tests.
+__device__ __forceinline__ bool scene_far(const DevEnv &E, float x, float y, float z, float rad) {
+    if (!E.field) return E.ns + E.nb + E.nc == 0;
+    const float ax = fmaxf(fmaxf(E.lox - x, x - E.hix), 0.f), ay = fmaxf(fmaxf(E.loy - y, y - E.hiy), 0.f),
+                az = fmaxf(fmaxf(E.loz - z, z - E.hiz), 0.f);
+    if (ax * ax + ay * ay + az * az > rad * rad) return true;
+    const int ix = min(max((int)((x - E.ox) * E.inv_h), 0), E.nx - 1), iy = min(max((int)((y - E.oy) * E.inv_h), 0), E.ny - 1),
+              iz = min(max((int)((z - E.oz) * E.inv_h), 0), E.nz - 1);
+    const float d = __ldg(E.field + ((iz * E.ny + iy) * E.nx + ix));
+    const float dx = x - (E.ox + ((float)ix + 0.5f) * E.h), dy = y - (E.oy + ((float)iy + 0.5f) * E.h),
+                dz = z - (E.oz + ((float)iz + 0.5f) * E.h);
+    return d - sqrtf(dx * dx + dy * dy + dz * dz) > rad;
 }
 
 // ---------------------------------------------------------------------------------

@@ -160,14 +160,17 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
                               unsigned char *ok, int *first_hit);
 }  // namespace gbmp
 
+namespace gbmp {
+// Distance field of a scene (gbmp_field.cu): region and cells from the bounding spheres
+// (4 doubles each), then the values, written to `field` on stream s.
+bool scene_field_plan(const std::vector<double> &bounds, DevEnv &E);
+cudaError_t scene_field_build(const DevEnv &E, float *field, cudaStream_t s);
+}  // namespace gbmp
+
 struct gbmp_env_s {
     int ns = 0, nb = 0, nc = 0;
-    float4 *d_words = nullptr;
+    float4 *d_words = nullptr;   // one allocation: the words, then the field
     std::vector<float4> h_words;
-    gbmp::DevEnv dev() const {
-        gbmp::DevEnv e;
-        e.ns = ns; e.nb = nb; e.nc = nc;
-        e.words = d_words;
-        return e;
-    }
+    gbmp::DevEnv view{};
+    gbmp::DevEnv dev() const { return view; }
 };

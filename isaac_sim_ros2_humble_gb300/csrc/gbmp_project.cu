@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     k_project(DevRobot R, ProjParams p, float *__restrict__ qall, long long n, float *__restrict__ task_cost,
               float *__restrict__ bound_cost) {
     extern __shared__ __align__(16) unsigned char smem[];
-    DevEnv E0{0, 0, 0, nullptr};
+    DevEnv E0{};
     SmemTables t = carve_tables(smem, R, 0);
     if (!stage_tables(R, E0, t, 0)) return;
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
@@ -394,7 +394,7 @@ using namespace gbmp;
 __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     k_space_jacobian(DevRobot R, const float *__restrict__ q, long long n, float *__restrict__ jac) {
     extern __shared__ __align__(16) unsigned char smem[];
-    DevEnv E0{0, 0, 0, nullptr};
+    DevEnv E0{};
     SmemTables t = carve_tables(smem, R, 0);
     if (!stage_tables(R, E0, t, 0)) return;
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
