@@ -318,9 +318,9 @@ def bench_plain(args, flush, fp32_peak):
            "e2e": {"value": n / (float(np.median(e2e_ms)) / 1e3), "unit": "configs/s",
                    "h2d_bytes_per_step": int(n * L * 4), "d2h_bytes_per_step": int(n + n * L * 64),
                    "ms_per_step": float(np.median(e2e_ms))},
-           "roofline": {"bound": "fp32", "kernel": "k_check_states", "unit": "TFLOP/s", "peak": fp32_peak,
+           "roofline": {"bound": "fp32", "kernel": "k_check_verdicts", "unit": "TFLOP/s", "peak": fp32_peak,
                         "achieved": exec_flops / (k_ms_per / 1e3) / 1e12 if k_ms_per > 0 else None,
-                        "achieved_is": "flops executed by k_check_states (counted in-kernel in an untimed step) / "
+                        "achieved_is": "flops executed by k_check_verdicts (counted in-kernel in an untimed step) / "
                                        "its device time",
                         "effective": n * flops_state / (k_ms_per / 1e3) / 1e12 if k_ms_per > 0 else None,
                         "effective_is": "reference-equivalent work (all pairs of every configuration) / its device "

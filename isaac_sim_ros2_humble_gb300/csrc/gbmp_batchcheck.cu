@@ -5,11 +5,12 @@
 // launches.  Here a descriptor table lists the requests (robot tables, scene, inputs,
 // outputs), and a second table splits their states into block-sized ranges; every block
 // stages the tables of its own request into shared memory (bulk asynchronous copies) and
-// checks its range, one warp per state, with the per-state routine of k_check_states
-// (check_state), so each request's outputs are bit-identical to a gbmp_check_states_fk
-// call of its own.  Shared memory is sized for the largest request; the spheres-per-lane
-// template covers the robot with the most spheres (smaller robots leave slots empty).
-#include "gbmp_internal.h"
+// checks its range with the routines of k_check_verdicts (several states a warp,
+// check_verdicts) or k_check_costs (one, check_state), so each request's outputs are
+// bit-identical to a gbmp_check_states_fk call of its own.  Shared memory is sized for the
+// largest request; the spheres-per-lane template of the costs covers the robot with the
+// most spheres (smaller robots leave slots empty).
+#include "gbmp_states_device.cuh"
 
 namespace gbmp {
 
@@ -27,9 +28,9 @@ struct CheckRange {
     long long lo, hi;
 };
 
-template <bool COST, int SPL>
+template <int SPL>
 __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
-    k_check_batch(const CheckTask *__restrict__ tasks, const CheckRange *__restrict__ ranges) {
+    k_batch_costs(const CheckTask *__restrict__ tasks, const CheckRange *__restrict__ ranges) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ CheckTask sT;
     __shared__ CheckRange sB;
@@ -47,8 +48,33 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (long long s = sB.lo + threadIdx.x / kWarp; s < sB.hi; s += kWarpsPerBlock)
-        check_state<COST, SPL>(t, R, E, w, sT.q, s, sT.n, sT.verdict, sT.costs, sT.total, sT.poses, sT.centers,
-                               lane);
+        check_state<true, SPL>(t, R, E, w, sT.q, s, sT.n, sT.verdict, sT.costs, sT.total, sT.poses, sT.centers, lane);
+}
+
+// `ks` states a warp at a time.  256 requests over 4 robots and 16 scenes, 1.57 million
+// states: 5.38 ms with one warp for each state, 1.53 ms now.
+template <bool CNT>
+__global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStatesWarps)
+    k_batch_verdicts(const CheckTask *__restrict__ tasks, const CheckRange *__restrict__ ranges, int ks) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ CheckTask sT;
+    __shared__ CheckRange sB;
+    if (threadIdx.x == 0) {
+        sB = ranges[blockIdx.x];
+        sT = tasks[sB.task];
+    }
+    __syncthreads();
+    const DevRobot &R = sT.R;
+    const DevEnv &E = sT.E;
+    const int nwords = env_words(E.ns, E.nb, E.nc);
+    SmemTables t = carve_tables(smem, R, nwords);
+    if (!stage_tables(R, E, t, nwords)) return;
+    const int warps = blockDim.x / kWarp, warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
+    const StatesScratch sc = carve_states(smem + smem_tables_bytes(R, nwords), R, ks, warp);
+    const int vec = (reinterpret_cast<unsigned long long>(sT.poses) & 15ull) == 0;
+    for (long long s = sB.lo + warp * ks; s < sB.hi; s += warps * ks)
+        check_verdicts<CNT>(t, R, E, sc, sT.q, s, (int)min((long long)ks, sB.hi - s), sT.verdict, sT.poses, sT.centers,
+                            vec, lane);
 }
 
 #define GBMP_BATCH_SPL_SWITCH(spl, ...)                    \
@@ -150,15 +176,18 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
     }
     auto *tasks = reinterpret_cast<CheckTask *>(b->h_buf);
     auto *ranges = reinterpret_cast<CheckRange *>(b->h_buf + b->ranges_off);
+    const bool cost = mode == GBMP_CHECK_COST;
     int nt = 0, spl = 1;
-    size_t smem = 0;
+    size_t smem = 0;   // of the costs' kernel, which also says which requests fit
+    size_t tables = 0;
+    DevRobot widest{};
     long long total = 0;
     unsigned long long *work = work_counter();
     for (int i = 0; i < n_reqs; ++i) {
         const gbmp_check_request &q = reqs[i];
         if (q.n == 0) continue;
         CheckTask &T = tasks[nt++];
-        T.R = q.robot->dev;
+        T.R = cost ? q.robot->dev : q.robot->dev_chunk;
         T.R.work = work;
         T.E = q.env->dev();
         T.q = q.d_q;
@@ -169,8 +198,11 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         T.poses = q.d_poses;
         T.centers = q.d_centers;
         spl = std::max(spl, T.R.spl);
-        smem = std::max(smem, smem_tables_bytes(T.R, env_words(T.E.ns, T.E.nb, T.E.nc)) +
-                                  smem_warp_bytes(T.R) * kWarpsPerBlock);
+        const int words = env_words(T.E.ns, T.E.nb, T.E.nc);
+        smem = std::max(smem, smem_tables_bytes(q.robot->dev, words) + smem_warp_bytes(q.robot->dev) * kWarpsPerBlock);
+        tables = std::max(tables, smem_tables_bytes(T.R, words));
+        widest.L = std::max(widest.L, T.R.L);
+        widest.G = std::max(widest.G, T.R.G);
         total += q.n;
     }
     if (nt == 0) return GBMP_OK;
@@ -188,52 +220,62 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         return GBMP_ERR_CAPACITY;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    gbmp_status st = GBMP_OK;
-    const bool cost = mode == GBMP_CHECK_COST;
-    GBMP_BATCH_SPL_SWITCH(spl, {
-        const void *fn = cost ? (const void *)k_check_batch<true, SPL> : (const void *)k_check_batch<false, SPL>;
-        st = ensure_smem_optin(fn);
-        if (st) return st;
-        int per_sm = 0;
-        GBMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kWarpsPerBlock * kWarp, smem));
-        if (per_sm < 1) per_sm = 1;
-        // states per block: about eight waves over all requests (measured 6.03 ms against
-        // 6.14 for four, 6.5 for two and 7.6 for one on the 256-request benchmark mix), at
-        // least four states a warp
-        const long long target = 8LL * per_sm * b->num_sms;
-        long long spb = (total + target - 1) / target;
-        spb = std::max<long long>(spb, 4 * kWarpsPerBlock);
-        spb = (spb + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
-        int nr = 0;
-        for (int ti = 0; ti < nt; ++ti)
-            for (long long lo = 0; lo < tasks[ti].n; lo += spb) {
-                if (nr == b->max_ranges) {
-                    set_error("check batch: more than %d block ranges", b->max_ranges);
-                    return GBMP_ERR_CAPACITY;
-                }
-                ranges[nr++] = CheckRange{ti, 0, lo, std::min(lo + spb, tasks[ti].n)};
-            }
-        // tasks and ranges in one copy (the ranges follow the tasks at ranges_off)
-        const size_t nbytes = b->ranges_off + sizeof(CheckRange) * (size_t)nr;
-        if (b->ranges_off > sizeof(CheckTask) * (size_t)nt) {
-            GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, sizeof(CheckTask) * (size_t)nt, cudaMemcpyHostToDevice, s));
-            GBMP_CUDA(cudaMemcpyAsync(b->d_buf + b->ranges_off, b->h_buf + b->ranges_off,
-                                      sizeof(CheckRange) * (size_t)nr, cudaMemcpyHostToDevice, s));
-        } else {
-            GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, nbytes, cudaMemcpyHostToDevice, s));
+    const void *fn = nullptr;
+    StatesShape sh{1, kWarpsPerBlock, 1, smem};
+    if (cost) {
+        GBMP_BATCH_SPL_SWITCH(spl, { fn = (const void *)k_batch_costs<SPL>; });
+    } else {
+        fn = work ? (const void *)k_batch_verdicts<true> : (const void *)k_batch_verdicts<false>;
+    }
+    gbmp_status st = ensure_smem_optin(fn);
+    if (st) return st;
+    if (cost) {
+        GBMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sh.per_sm, fn, kWarpsPerBlock * kWarp, smem));
+        if (sh.per_sm < 1) sh.per_sm = 1;
+    } else {
+        // one shape for all requests: the largest tables, and the scratch of a warp of as many
+        // links and groups as any has
+        const size_t limit = kSmemLimit - sizeof(CheckTask) - sizeof(CheckRange) - 16;
+        const long long resident = (long long)kStatesResident * b->num_sms;
+        const int want = (int)std::min<long long>(kStatesKs, (total + resident - 1) / resident);
+        if (!states_shape(tables, [&](int ks) { return smem_states_bytes(widest, ks); }, want, limit, &sh)) {
+            set_error("check batch: the largest request needs %zu bytes of shared memory", smem);
+            return GBMP_ERR_CAPACITY;
         }
-        GBMP_CUDA(cudaEventRecord(b->uploaded, s));
-        b->pending = true;
-        const auto *d_tasks = reinterpret_cast<const CheckTask *>(b->d_buf);
-        const auto *d_ranges = reinterpret_cast<const CheckRange *>(b->d_buf + b->ranges_off);
-        ProfScope ps(GBMP_PROF_CHECK_STATES, s);
-        if (cost)
-            k_check_batch<true, SPL><<<nr, kWarpsPerBlock * kWarp, smem, s>>>(d_tasks, d_ranges);
-        else
-            k_check_batch<false, SPL><<<nr, kWarpsPerBlock * kWarp, smem, s>>>(d_tasks, d_ranges);
-    });
-    GBMP_CUDA(cudaGetLastError());
-    return st;
+    }
+    // states per block: about eight waves over all requests (1.53 ms on the 256-request mix
+    // above; four: 1.57, sixteen: 1.52), at least one round of its warps
+    const long long unit = (long long)sh.warps * sh.ks;
+    const long long target = (long long)std::min(8 * sh.per_sm, kBatchBlocksPerSm) * b->num_sms;
+    long long spb = (total + target - 1) / target;
+    spb = std::max<long long>(spb, cost ? 4 * unit : unit);   // costs: at least four states a warp
+    spb = (spb + unit - 1) / unit * unit;
+    int nr = 0;
+    for (int ti = 0; ti < nt; ++ti)
+        for (long long lo = 0; lo < tasks[ti].n; lo += spb) {
+            if (nr == b->max_ranges) {
+                set_error("check batch: more than %d block ranges", b->max_ranges);
+                return GBMP_ERR_CAPACITY;
+            }
+            ranges[nr++] = CheckRange{ti, 0, lo, std::min(lo + spb, tasks[ti].n)};
+        }
+    // tasks and ranges in one copy (the ranges follow the tasks at ranges_off)
+    const size_t nbytes = b->ranges_off + sizeof(CheckRange) * (size_t)nr;
+    if (b->ranges_off > sizeof(CheckTask) * (size_t)nt) {
+        GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, sizeof(CheckTask) * (size_t)nt, cudaMemcpyHostToDevice, s));
+        GBMP_CUDA(cudaMemcpyAsync(b->d_buf + b->ranges_off, b->h_buf + b->ranges_off, sizeof(CheckRange) * (size_t)nr,
+                                  cudaMemcpyHostToDevice, s));
+    } else {
+        GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, nbytes, cudaMemcpyHostToDevice, s));
+    }
+    GBMP_CUDA(cudaEventRecord(b->uploaded, s));
+    b->pending = true;
+    const auto *d_tasks = reinterpret_cast<const CheckTask *>(b->d_buf);
+    const auto *d_ranges = reinterpret_cast<const CheckRange *>(b->d_buf + b->ranges_off);
+    ProfScope ps(GBMP_PROF_CHECK_STATES, s);
+    void *args[] = {&d_tasks, &d_ranges, &sh.ks};   // the costs' kernel takes the first two
+    GBMP_CUDA(cudaLaunchKernel(fn, dim3(nr), dim3(sh.warps * kWarp), args, sh.smem, s));
+    return GBMP_OK;
 }
 
 }  // extern "C"

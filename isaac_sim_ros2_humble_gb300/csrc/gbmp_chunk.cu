@@ -1,8 +1,8 @@
 // gbmp_chunk.cu -- the edge-validation kernel (one warp per edge, the edge's states in
 // chunks of consecutive states; the chunk routines are in gbmp_chunk_device.cuh), its
 // launch set-up, and FK alone by chunks of consecutive states (gbmp_fk).
-#include "gbmp_chunk_device.cuh"
 #include "gbmp_order.h"
+#include "gbmp_states_device.cuh"
 
 namespace gbmp {
 
@@ -182,33 +182,7 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
         const int ks = (int)min((long long)kFkChunk, n - s0);
         const float *qc = q + s0 * L;
         warp_fk_chunk_q<kFkChunk>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, lpK, lane);
-        if (poses) {
-            if (vec) {
-                float4 *P4 = reinterpret_cast<float4 *>(poses + s0 * L * 16);
-                const float4 *rows = reinterpret_cast<const float4 *>(lpK);
-                for (int f = lane; f < ks * L * 4; f += kWarp) {
-                    const int r = f & 3, kl = f >> 2;   // kl = k * L + link
-                    P4[f] = r < 3 ? rows[3 * kl + r] : make_float4(0.f, 0.f, 0.f, 1.f);
-                }
-            } else {
-                float *P = poses + s0 * L * 16;
-                for (int e = lane; e < ks * L * 16; e += kWarp) {
-                    const int kl = e >> 4, k = e & 15;
-                    P[e] = k < 12 ? lpK[12 * kl + k] : (k == 15 ? 1.f : 0.f);
-                }
-            }
-        }
-        if (centers) {
-            float *Cc = centers + s0 * S * 3;
-            for (int p = lane; p < ks * S; p += kWarp) {
-                const int k = p / S, j = p - k * S;
-                const float4 sp = t.sph[j];
-                const float3 c3 = xform_point_a16(lpK + 12 * (k * L + t.slink[j]), sp.x, sp.y, sp.z);
-                Cc[3 * p] = c3.x;
-                Cc[3 * p + 1] = c3.y;
-                Cc[3 * p + 2] = c3.z;
-            }
-        }
+        store_fk_states(t, L, S, lpK, s0, ks, poses, centers, vec, lane);
         __syncwarp();
     }
 }

@@ -70,8 +70,9 @@ __device__ inline void carve_chunk(unsigned char *base, const DevRobot &R, int K
 // k.  The arithmetic is warp_fk's (joint_local, mul_elem), so poses are bit-identical.
 template <int K, typename QV>
 __device__ inline void warp_fk_chunk_q(const SmemTables &t, int L, int ks, QV qv, float *lpK, int lane) {
+    const unsigned rks = (65536u + ks - 1u) / ks;   // idx / ks = idx * rks >> 16 (idx < 64 * 10)
     for (int idx = lane; idx < ks * (L - 1); idx += kWarp) {
-        const int i = 1 + idx / ks, k = idx - (i - 1) * ks;
+        const int i = 1 + (int)(idx * rks >> 16), k = idx - (i - 1) * ks;
         joint_local(t, i, qv(k, i), lpK + 12 * (k * L + i));
     }
     __syncwarp();
@@ -155,10 +156,10 @@ __device__ __forceinline__ float3 xform_point_a16(const float *T, float x, float
     return o;
 }
 
-// Sphere k's centre in the state whose link poses start at lp.
-__device__ __forceinline__ float3 sphere_centre(const SmemTables &t, const float *lp, int k, float4 &s) {
-    s = t.sph[k];
-    return xform_point_a16(lp + 12 * t.slink[k], s.x, s.y, s.z);
+// Sphere j's centre in a state; T is the pose of its link.
+__device__ __forceinline__ float3 sphere_centre(const SmemTables &t, const float *T, int j, float4 &s) {
+    s = t.sph[j];
+    return xform_point_a16(T, s.x, s.y, s.z);
 }
 
 // Group g's bounding sphere in the state whose link poses start at lp.
@@ -192,11 +193,12 @@ __device__ __forceinline__ int chunk_obstacle(const SmemTables &t, const DevRobo
     for (; gm; gm &= gm - 1u) {
         const int g = __ffs(gm) - 1;
         const int g0 = t.gso[g], ng = t.gso[g + 1] - g0, total = ng * kmax;
+        const float *T = lpK + 12 * t.glink[g];
         const float inv = 1.f / (float)ng;
         for (int idx = lane; idx < total; idx += kWarp) {
             const int k = (int)(((float)idx + 0.5f) * inv);   // idx / ng (idx < 2^12)
             float4 s;
-            const float3 c = sphere_centre(t, lpK + k * 12 * R.L, t.gsl[g0 + idx - k * ng], s);
+            const float3 c = sphere_centre(t, T + k * 12 * R.L, g0 + idx - k * ng, s);
             bool h;
             if (TYPE == 0) {   // expanded form, see warp_collide
                 const float A = __fmaf_rn(c.z, c.z, __fmaf_rn(c.y, c.y, __fmaf_rn(c.x, c.x, -s.w * s.w)));
@@ -225,15 +227,68 @@ __device__ __forceinline__ int chunk_obstacle(const SmemTables &t, const DevRobo
     return hk;
 }
 
-// Self pairs of the group pairs cs.pl[0 .. npr) in the states k < kmax.  The lanes first
+// Whether a sphere of one group touches one of the other, eight lanes for a group pair
+// (sl the lane's place among them, sh its first lane's number; every warp settles four
+// pairs at once; pr: the pair's word of lpair, all 0 for none): the spheres of b against
+// a's group sphere GA, and only where one touches it, a's spheres against GB and the
+// touching pairs exactly, with the pair threshold (ri + rj)^2 rounded as the pair list's.
+// A sphere that touches a sphere of the other group touches that group's enclosing sphere,
+// so nothing is lost.  A group pair whose enabled sphere pairs are not all (sphere of a,
+// sphere of b) pairs walks the pair list.  lp: the state's link poses.  True on the lanes
+// that found a contact.
+template <bool CNT>
+__device__ __forceinline__ bool group_pair_hits(const SmemTables &t, const DevRobot &R, const float *lp, int4 pr,
+                                                float4 GA, float4 GB, int sl, int sh, unsigned long long &fl) {
+    bool hit = false;
+    const int na = pair_count(pr.x), nb = pair_count(pr.y), b0 = pair_first(pr.y);
+    const bool full = pr.w - pr.z == na * nb;
+    const float *TA = lp + 12 * t.glink[pair_group(pr.x)], *TB = lp + 12 * t.glink[pair_group(pr.y)];
+    const int nbw = __reduce_max_sync(kFull, full ? nb : 0);
+    for (int jb = 0; jb < nbw; jb += 8) {
+        bool ib = false;
+        if (full && jb + sl < nb) {
+            float4 s;
+            const float3 c = sphere_centre(t, TB, b0 + jb + sl, s);
+            const float rr = s.w + GA.w;
+            ib = sq3(c.x - GA.x, c.y - GA.y, c.z - GA.z) < rr * rr;
+        }
+        const unsigned mb = (__ballot_sync(kFull, ib) >> sh) & 0xffu;
+        if (mb) {
+            for (int ja = sl; ja < na; ja += 8) {
+                float4 s;
+                const float3 c = sphere_centre(t, TA, pair_first(pr.x) + ja, s);
+                const float rr = s.w + GB.w;
+                if (sq3(c.x - GB.x, c.y - GB.y, c.z - GB.z) < rr * rr) {
+                    for (unsigned m = mb; m; m &= m - 1u) {
+                        float4 sb;
+                        const float3 cb = sphere_centre(t, TB, b0 + jb + __ffs(m) - 1, sb);
+                        const float sr = __fadd_rn(s.w, sb.w);
+                        hit |= sq3(c.x - cb.x, c.y - cb.y, c.z - cb.z) < __fmul_rn(sr, sr);
+                    }
+                }
+            }
+        }
+        if (CNT) {   // sphere centres and tests against the group spheres
+            fl += (unsigned long long)__popc(__ballot_sync(kFull, full && jb + sl < nb)) * (18 + kFlSelf);
+            fl += (unsigned long long)__reduce_add_sync(kFull, sl == 0 && mb ? na : 0) * (18 + kFlSelf);
+        }
+    }
+    if (!full)
+        for (int p = pr.z + sl; p < pr.w; p += 8) {
+            const unsigned ij = __ldg(R.pairs + p);
+            const float thr = __ldg(R.thr + p);
+            float4 s;
+            const float3 a = sphere_centre(t, lp + 12 * t.slink[ij & 0xffffu], ij & 0xffffu, s),
+                         b = sphere_centre(t, lp + 12 * t.slink[ij >> 16], ij >> 16, s);
+            hit |= sq3(a.x - b.x, a.y - b.y, a.z - b.z) < thr;
+        }
+    return hit;
+}
+
+// Self pairs of the group pairs cs.pl[0 .. npr) in the states k < kmax: the lanes first
 // take (state, pair) items and keep those whose group spheres overlap; the kept items are
-// settled four at a time, eight lanes each: b's spheres against a's group sphere, and
-// only where one touches it, a's spheres against b's group sphere and the touching pairs
-// exactly, with the pair threshold (ri + rj)^2 rounded as the pair list's.  A sphere that
-// touches a sphere of the other group touches that group's enclosing sphere, so nothing
-// is lost.  A group pair whose enabled sphere pairs are not all (sphere of a, sphere of
-// b) pairs walks its range of the pair list.  Returns the lane's lowest colliding state,
-// or kmax.
+// settled four at a time (group_pair_hits).  Returns the lane's lowest colliding state, or
+// kmax.
 template <bool CNT>
 __device__ __forceinline__ int chunk_self(const SmemTables &t, const DevRobot &R, const ChunkScratch &cs, int npr,
                                           int kmax, bool any, int lane, unsigned long long &fl) {
@@ -248,7 +303,8 @@ __device__ __forceinline__ int chunk_self(const SmemTables &t, const DevRobot &R
         if (idx < total) {
             const int k = (int)(((float)idx + 0.5f) * inv), p = cs.pl[idx - k * npr];   // idx / npr (idx < 2^12)
             const int4 lp = t.lpair[p];
-            const float4 a = group_sphere(t, cs.lpK + k * 12 * R.L, lp.x), b = group_sphere(t, cs.lpK + k * 12 * R.L, lp.y);
+            const float *poses = cs.lpK + k * 12 * R.L;
+            const float4 a = group_sphere(t, poses, pair_group(lp.x)), b = group_sphere(t, poses, pair_group(lp.y));
             const float rr = a.w + b.w;
             on = sq3(a.x - b.x, a.y - b.y, a.z - b.z) < rr * rr;
             item = (p << 5) | k;
@@ -260,59 +316,19 @@ __device__ __forceinline__ int chunk_self(const SmemTables &t, const DevRobot &R
         __syncwarp();
         const int nit = __popc(bal);
         for (int j0 = 0; j0 < nit; j0 += 4) {
-            int k = 0, a0 = 0, na = 0, b0 = 0, nb = 0, p0 = 0, np = 0;
+            int k = 0;
+            int4 pr = make_int4(0, 0, 0, 0);
             float4 GA = make_float4(0.f, 0.f, 0.f, 0.f), GB = GA;
             const float *lp = cs.lpK;
             if (j0 + sub < nit) {
                 const int v = cs.it[j0 + sub];
                 k = v & 31;
-                const int4 q = t.lpair[v >> 5];
+                pr = t.lpair[v >> 5];
                 lp += k * 12 * R.L;
-                a0 = t.gso[q.x]; na = t.gso[q.x + 1] - a0;
-                b0 = t.gso[q.y]; nb = t.gso[q.y + 1] - b0;
-                p0 = q.z; np = q.w - q.z;
-                GA = group_sphere(t, lp, q.x);
-                GB = group_sphere(t, lp, q.y);
+                GA = group_sphere(t, lp, pair_group(pr.x));
+                GB = group_sphere(t, lp, pair_group(pr.y));
             }
-            const bool full = np == na * nb;
-            const int nbw = __reduce_max_sync(kFull, full ? nb : 0);
-            for (int jb = 0; jb < nbw; jb += 8) {
-                bool ib = false;
-                if (full && jb + sl < nb) {
-                    float4 s;
-                    const float3 c = sphere_centre(t, lp, t.gsl[b0 + jb + sl], s);
-                    const float rr = s.w + GA.w;
-                    ib = sq3(c.x - GA.x, c.y - GA.y, c.z - GA.z) < rr * rr;
-                }
-                const unsigned mb = (__ballot_sync(kFull, ib) >> sh) & 0xffu;
-                if (mb) {
-                    for (int ja = sl; ja < na; ja += 8) {
-                        float4 s;
-                        const float3 c = sphere_centre(t, lp, t.gsl[a0 + ja], s);
-                        const float rr = s.w + GB.w;
-                        if (sq3(c.x - GB.x, c.y - GB.y, c.z - GB.z) < rr * rr) {
-                            for (unsigned m = mb; m; m &= m - 1u) {
-                                float4 sb;
-                                const float3 cb = sphere_centre(t, lp, t.gsl[b0 + jb + __ffs(m) - 1], sb);
-                                const float sr = __fadd_rn(s.w, sb.w);
-                                if (sq3(c.x - cb.x, c.y - cb.y, c.z - cb.z) < __fmul_rn(sr, sr)) hk = min(hk, k);
-                            }
-                        }
-                    }
-                }
-                if (CNT) {   // sphere centres and tests against the group spheres
-                    fl += (unsigned long long)__popc(__ballot_sync(kFull, full && jb + sl < nb)) * (18 + kFlSelf);
-                    fl += (unsigned long long)__reduce_add_sync(kFull, sl == 0 && mb ? na : 0) * (18 + kFlSelf);
-                }
-            }
-            if (!full)
-                for (int p = p0 + sl; p < p0 + np; p += 8) {
-                    const unsigned ij = __ldg(R.pairs + p);
-                    const float thr = __ldg(R.thr + p);
-                    float4 s;
-                    const float3 a = sphere_centre(t, lp, ij & 0xffffu, s), b = sphere_centre(t, lp, ij >> 16, s);
-                    if (sq3(a.x - b.x, a.y - b.y, a.z - b.z) < thr) hk = min(hk, k);
-                }
+            if (group_pair_hits<CNT>(t, R, lp, pr, GA, GB, sl, sh, fl)) hk = min(hk, k);
             if (any && __any_sync(kFull, hk < kmax)) return hk;
         }
         __syncwarp();
@@ -465,7 +481,7 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
         bool on = false;
         if (k < R.NPL) {
             const int4 lpr = t.lpair[k];
-            const float4 a = cs.sgb[lpr.x], b = cs.sgb[lpr.y];
+            const float4 a = cs.sgb[pair_group(lpr.x)], b = cs.sgb[pair_group(lpr.y)];
             const float rr = a.w + b.w;
             on = sq3(a.x - b.x, a.y - b.y, a.z - b.z) < rr * rr;
         }

@@ -8,6 +8,7 @@
 #include "gbmp_groups.h"
 #include "gbmp_internal.h"
 #include "gbmp_order.h"
+#include "gbmp_states_device.cuh"
 
 namespace gbmp {
 
@@ -86,16 +87,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     }
 }
 
-// Collision check of n states; one warp per state.  With poses / centers non-null the
-// FK of each state is also written out (the reference's update() and checkStates() from
-// one FK).  Four blocks per SM (64 registers): 4,096 states then take one round of the
-// resident warps (4,864) instead of two of 3,648 (measured 16.3 against 18.4 us on the
-// plain 4,096-configuration workload).
-template <bool COST, int SPL>
+// Costs of n states; one warp per state.  With poses / centers non-null the FK of each
+// state is also written out (the reference's update() and checkStates() from one FK).
+template <int SPL>
 __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
-    k_check_states(DevRobot R, DevEnv E, const float *__restrict__ q, long long n,
-                   unsigned char *__restrict__ verdict, float *__restrict__ costs, float *__restrict__ total,
-                   float *__restrict__ poses, float *__restrict__ centers) {
+    k_check_costs(DevRobot R, DevEnv E, const float *__restrict__ q, long long n, unsigned char *__restrict__ verdict,
+                  float *__restrict__ costs, float *__restrict__ total, float *__restrict__ poses,
+                  float *__restrict__ centers) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nwords = env_words(E.ns, E.nb, E.nc);
     SmemTables t = carve_tables(smem, R, nwords);
@@ -105,7 +103,27 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
     const int lane = threadIdx.x & 31;
     const long long nw = (long long)gridDim.x * kWarpsPerBlock;
     for (long long s = blockIdx.x * (long long)kWarpsPerBlock + threadIdx.x / kWarp; s < n; s += nw)
-        check_state<COST, SPL>(t, R, E, w, q, s, n, verdict, costs, total, poses, centers, lane);
+        check_state<true, SPL>(t, R, E, w, q, s, n, verdict, costs, total, poses, centers, lane);
+}
+
+// Collision verdicts of n states, `ks` states a warp at a time (gbmp_states_device.cuh).
+// One warp for each state, testing every obstacle against every group sphere, took 14.4 us
+// for the 4,096 configurations of the plain workload with their poses (12.3 us now), 250 us
+// for 70,072 states of a 9-DOF arm in 223 obstacles (75 us).
+template <bool CNT>
+__global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStatesWarps)
+    k_check_verdicts(DevRobot R, DevEnv E, const float *__restrict__ q, long long n, int ks,
+                     unsigned char *__restrict__ verdict, float *__restrict__ poses, float *__restrict__ centers,
+                     int vec) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nwords = env_words(E.ns, E.nb, E.nc);
+    SmemTables t = carve_tables(smem, R, nwords);
+    if (!stage_tables(R, E, t, nwords)) return;
+    const int warps = blockDim.x / kWarp, warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
+    const StatesScratch sc = carve_states(smem + smem_tables_bytes(R, nwords), R, ks, warp);
+    const long long step = (long long)gridDim.x * warps * ks;
+    for (long long s = ((long long)blockIdx.x * warps + warp) * ks; s < n; s += step)
+        check_verdicts<CNT>(t, R, E, sc, q, s, (int)min((long long)ks, n - s), verdict, poses, centers, vec, lane);
 }
 
 // Edge set-up: step count, direction, L2 length (KernelGenerator.h:433-465); one thread per
@@ -370,30 +388,51 @@ static gbmp_status pack_tables(gbmp_robot_s *r, int piece, void **block, DevRobo
     split_sphere_groups(L, S, r->slink.data(), r->sph_pos.data(), piece, piece > 0 ? std::min(kMaxGroups, 3 * L) : 0,
                         glink, sgrp);
     const int G = (int)glink.size();
+    // Pieces of links: the spheres in group order, so that a group's spheres are
+    // sph[gso[g]] .. sph[gso[g + 1] - 1].  place: where each sphere of the description stands.
+    std::vector<int> place(S ? S : 1, 0), slink(r->slink), pairs(r->pairs);
+    for (int k = 0; k < S; ++k) place[k] = k;
+    if (piece > 0) {
+        std::vector<int> by(S);
+        for (int k = 0; k < S; ++k) by[k] = k;
+        std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return sgrp[x] < sgrp[y]; });
+        const std::vector<float> sph0(sph);
+        const std::vector<int> sgrp0(sgrp);
+        for (int i = 0; i < S; ++i) {
+            place[by[i]] = i;
+            for (int a = 0; a < 4; ++a) sph[4 * i + a] = sph0[4 * by[i] + a];
+            slink[i] = r->slink[by[i]];
+            sgrp[i] = sgrp0[by[i]];
+        }
+        for (int &v : pairs) v = place[v];
+    }
     std::vector<float> grp(4 * (G ? G : 1), 0.f);
     for (int g = 0; g < G; ++g) {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int k = 0; k < S; ++k)
             if (sgrp[k] == g)
                 for (int a = 0; a < 3; ++a) {
-                    lo[a] = std::min(lo[a], (double)r->sph_pos[3 * k + a] - r->sph_r[k]);
-                    hi[a] = std::max(hi[a], (double)r->sph_pos[3 * k + a] + r->sph_r[k]);
+                    lo[a] = std::min(lo[a], (double)sph[4 * k + a] - sph[4 * k + 3]);
+                    hi[a] = std::max(hi[a], (double)sph[4 * k + a] + sph[4 * k + 3]);
                 }
         double c[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])}, rad = 0.0;
         for (int k = 0; k < S; ++k)
             if (sgrp[k] == g) {
                 double d2 = 0.0;
-                for (int a = 0; a < 3; ++a) d2 += (r->sph_pos[3 * k + a] - c[a]) * (r->sph_pos[3 * k + a] - c[a]);
-                rad = std::max(rad, std::sqrt(d2) + r->sph_r[k]);
+                for (int a = 0; a < 3; ++a) d2 += (sph[4 * k + a] - c[a]) * (sph[4 * k + a] - c[a]);
+                rad = std::max(rad, std::sqrt(d2) + sph[4 * k + 3]);
             }
         for (int a = 0; a < 3; ++a) grp[4 * g + a] = (float)c[a];
         grp[4 * g + 3] = nextafterf((float)(rad + kBroadMargin), 1e30f);
     }
+    std::vector<int> gso(G + 1, 0);   // first sphere of each group, counted in group order
+    for (int k = 0; k < S; ++k) gso[sgrp[k] + 1]++;
+    for (int g = 0; g < G; ++g) gso[g + 1] += gso[g];
     // Device pair list sorted by group pair; each enabled group pair owns a range.
     std::vector<int> order(r->P);
     for (int p = 0; p < r->P; ++p) order[p] = p;
     auto key = [&](int p) {
-        const int a = sgrp[r->pairs[2 * p]], b = sgrp[r->pairs[2 * p + 1]];
+        const int a = sgrp[pairs[2 * p]], b = sgrp[pairs[2 * p + 1]];
         return std::make_pair(std::min(a, b), std::max(a, b));
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return key(x) < key(y); });
@@ -402,31 +441,25 @@ static gbmp_status pack_tables(gbmp_robot_s *r, int piece, void **block, DevRobo
     std::vector<int> lpair;
     for (int q = 0; q < r->P; ++q) {
         const int p = order[q];
-        packed[q] = (unsigned)r->pairs[2 * p] | ((unsigned)r->pairs[2 * p + 1] << 16);
+        packed[q] = (unsigned)pairs[2 * p] | ((unsigned)pairs[2 * p + 1] << 16);
         thr_sorted[q] = r->thr[p];
         if (q == 0 || key(p) != key(order[q - 1])) {
-            lpair.insert(lpair.end(), {key(p).first, key(p).second, q, q});
+            auto word = [&](int g) { return g | gso[g] << 8 | (gso[g + 1] - gso[g]) << 17; };   // pair_group ...
+            lpair.insert(lpair.end(), {word(key(p).first), word(key(p).second), q, q});
         }
         lpair.back() = q + 1;
     }
     const int NPL = (int)lpair.size() / 4;
-    std::vector<int> gso(G + 1, 0), gsl(S ? S : 1, 0);   // spheres of each group, index order
-    for (int k = 0; k < S; ++k) gso[sgrp[k] + 1]++;
-    for (int g = 0; g < G; ++g) gso[g + 1] += gso[g];
-    {
-        std::vector<int> fill(gso.begin(), gso.end() - 1);
-        for (int k = 0; k < S; ++k) gsl[fill[sgrp[k]]++] = k;
-    }
     // The tables the kernels stage in shared memory come first, segment for segment in
     // the order and 16-byte alignment of carve_tables, so that one bulk copy of
     // smem_tables_bytes(R, 0) bytes stages them; the tables read from global memory follow.
     size_t o_jl = put(jl.data(), jl.size() * 4), o_axn = put(axn.data(), axn.size() * 4);
     size_t o_axr = put(axr.data(), axr.size() * 4), o_sph = put(sph.data(), 4 * 4 * (size_t)S);
     size_t o_type = put(r->type.data(), 4 * L), o_par = put(r->parent.data(), 4 * L);
-    size_t o_sl = put(r->slink.data(), 4 * (size_t)S);
+    size_t o_sl = put(slink.data(), 4 * (size_t)S);
     size_t o_grp = put(grp.data(), 4 * 4 * (size_t)G), o_glink = put(glink.data(), 4 * (size_t)G);
     size_t o_sgrp = put(sgrp.data(), 4 * (size_t)S), o_lpair = put(lpair.data(), 4 * lpair.size());
-    size_t o_gso = put(gso.data(), 4 * (size_t)(G + 1)), o_gsl = put(gsl.data(), 4 * (size_t)S);
+    size_t o_gso = put(gso.data(), 4 * (size_t)(G + 1)), o_place = put(place.data(), 4 * (size_t)S);
     const size_t staged_bytes = align16(blob.size());
     size_t o_pairs = put(packed.data(), 4 * (size_t)r->P), o_thr = put(thr_sorted.data(), 4 * (size_t)r->P);
     size_t o_lo = put(r->lower.data(), 4 * L), o_up = put(r->upper.data(), 4 * L);
@@ -457,7 +490,7 @@ static gbmp_status pack_tables(gbmp_robot_s *r, int piece, void **block, DevRobo
     }
     D.grp = (const float *)(b + o_grp); D.glink = (const int *)(b + o_glink);
     D.sgrp = (const int *)(b + o_sgrp); D.lpair = (const int4 *)(b + o_lpair);
-    D.gso = (const int *)(b + o_gso); D.gsl = (const int *)(b + o_gsl);
+    D.gso = (const int *)(b + o_gso); D.place = (const int *)(b + o_place);
     D.stage = b;
     D.stage_bytes = (unsigned)staged_bytes;
     D.fault = (unsigned *)(b + o_fault);
@@ -755,11 +788,11 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     bound(cc, crd);
     const bool field = scene_field_plan(bounds, E);
     const size_t wbytes = sizeof(float4) * e->h_words.size();
-    cudaError_t err = cudaMalloc(&e->d_words, wbytes + (field ? sizeof(float) * (size_t)E.nx * E.ny * E.nz : 0));
+    cudaError_t err = cudaMalloc(&e->d_words, wbytes + (field ? sizeof(float4) * (size_t)E.nx * E.ny * E.nz : 0));
     if (err == cudaSuccess) err = cudaMemcpy(e->d_words, e->h_words.data(), wbytes, cudaMemcpyHostToDevice);
     E.words = e->d_words;
     if (err == cudaSuccess && field) {
-        float *values = reinterpret_cast<float *>(e->d_words + e->h_words.size());
+        float4 *values = e->d_words + e->h_words.size();
         err = scene_field_build(E, values, nullptr);
         if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
         E.field = values;
@@ -819,30 +852,50 @@ gbmp_status gbmp_check_states_fk(gbmp_robot r, gbmp_env env, const float *d_q, i
     if (n == 0) return GBMP_OK;
     GBMP_CHECK_ARG(d_q, "q is NULL");
     const DevEnv E = env->dev();
-    DevRobot D = r->dev;
-    D.work = work_counter();
-    const size_t smem = block_smem(D, env_words(E.ns, E.nb, E.nc));
-    const long long need = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    gbmp_status st = GBMP_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    GBMP_SPL_SWITCH(r->dev.spl, {
-        int grid = 0;
-        if (mode == GBMP_CHECK_COST) {
-            st = persistent_grid(k_check_states<true, SPL>, smem, r->num_sms, &grid);
+    const int nwords = env_words(E.ns, E.nb, E.nc);
+    gbmp_status st = GBMP_OK;
+    if (mode == GBMP_CHECK_COST) {
+        DevRobot D = r->dev;
+        D.work = work_counter();
+        const size_t smem = block_smem(D, nwords);
+        const long long need = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
+        GBMP_SPL_SWITCH(r->dev.spl, {
+            int grid = 0;
+            st = persistent_grid(k_check_costs<SPL>, smem, r->num_sms, &grid);
             if (st) return st;
             if (need < grid) grid = (int)need;
             ProfScope ps(GBMP_PROF_CHECK_STATES, s);
-            k_check_states<true, SPL><<<grid, kWarpsPerBlock * kWarp, smem, s>>>(D, E, d_q, n, d_verdict, d_costs,
-                                                                                 d_total, d_poses, d_centers);
-        } else {
-            st = persistent_grid(k_check_states<false, SPL>, smem, r->num_sms, &grid);
-            if (st) return st;
-            if (need < grid) grid = (int)need;
-            ProfScope ps(GBMP_PROF_CHECK_STATES, s);
-            k_check_states<false, SPL><<<grid, kWarpsPerBlock * kWarp, smem, s>>>(D, E, d_q, n, d_verdict, nullptr,
-                                                                                  nullptr, d_poses, d_centers);
-        }
-    });
+            k_check_costs<SPL><<<grid, kWarpsPerBlock * kWarp, smem, s>>>(D, E, d_q, n, d_verdict, d_costs, d_total,
+                                                                          d_poses, d_centers);
+        });
+        GBMP_CUDA(cudaGetLastError());
+        return GBMP_OK;
+    }
+    DevRobot D = r->dev_chunk;
+    D.work = work_counter();
+    auto kern = D.work ? k_check_verdicts<true> : k_check_verdicts<false>;
+    st = ensure_smem_optin((const void *)kern);
+    if (st) return st;
+    const long long resident = (long long)kStatesResident * r->num_sms;
+    const int want = (int)std::min<long long>(kStatesKs, (n + resident - 1) / resident);
+    StatesShape sh;
+    if (block_smem(r->dev, nwords) > kSmemLimit ||
+        !states_shape(smem_tables_bytes(D, nwords), [&](int ks) { return smem_states_bytes(D, ks); }, want, kSmemLimit, &sh)) {
+        set_error("kernel does not fit on an SM (%zu bytes of shared memory)", block_smem(r->dev, nwords));
+        return GBMP_ERR_CAPACITY;
+    }
+    // few states: fewer warps a block, on more SMs (58 states in four blocks: 13.4 us, 9.4 us
+    // with a block for each state)
+    while (sh.warps > 1 && (n + sh.ks * sh.warps - 1) / (sh.ks * sh.warps) < r->num_sms) {
+        sh.warps /= 2;
+        sh.smem = smem_tables_bytes(D, nwords) + smem_states_bytes(D, sh.ks) * sh.warps;
+    }
+    const long long need = (n + sh.ks * sh.warps - 1) / (sh.ks * sh.warps);
+    const int grid = (int)std::min<long long>(need, (long long)sh.per_sm * r->num_sms);
+    const int vec = (reinterpret_cast<uintptr_t>(d_poses) & 15u) == 0;
+    ProfScope ps(GBMP_PROF_CHECK_STATES, s);
+    kern<<<grid, sh.warps * kWarp, sh.smem, s>>>(D, E, d_q, n, sh.ks, d_verdict, d_poses, d_centers, vec);
     GBMP_CUDA(cudaGetLastError());
     return GBMP_OK;
 }

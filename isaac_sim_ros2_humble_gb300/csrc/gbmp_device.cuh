@@ -34,8 +34,11 @@ constexpr float kFar = 1.0e15f;           // parking spot for unused sphere slot
 //         link pair so that each enabled link pair owns a contiguous range
 //   grp   [G*4]  per sphere-carrying link ("group"): bounding sphere (x, y, z, R) in the
 //         link frame enclosing all its spheres, inflated by kBroadMargin
-//   glink [G], sgrp [S] (group of each sphere), lpair [NPL*4] (ga, gb, p0, p1)
-//   gso [G+1], gsl [S]: the spheres of group g are gsl[gso[g] .. gso[g+1]) in index order
+//   glink [G], sgrp [S] (group of each sphere), lpair [NPL*4] (a, b, p0, p1): two groups
+//         (pair_group, pair_first, pair_count) and their range of the pair list
+//   gso [G+1]: first sphere of each group, in group order; place [S]: where each sphere of
+//         the description stands in sph (itself, or in group order for the groups that are
+//         pieces of links, whose spheres are then sph[gso[g] .. gso[g+1]))
 // Environment words (float4):
 //   spheres  [ns]     (x, y, z, r)
 //   cuboids  [nb*5]   inverse pose rows 0..2, (min xyz, 0), (max xyz, 0)
@@ -59,12 +62,12 @@ struct DevRobot {
     const float *grp;
     const int *glink, *sgrp;
     const int4 *lpair;
-    const int *gso, *gsl;
+    const int *gso, *place;
     // Executed-work accounting (only when `work` is non-null): work[0] += flops executed,
     // work[1] += states evaluated.  base_flops = per-state FK + sphere + group transforms.
     unsigned long long *work;
     long long base_flops;
-    // The staged tables (jl .. gsl above) as one block laid out exactly as carve_tables
+    // The staged tables (jl .. place above) as one block laid out exactly as carve_tables
     // lays them out in shared memory: `stage_bytes` bytes at `stage` (16-byte aligned), so
     // that one bulk copy stages them.  `fault`: device word a kernel sets (bit 0) when a
     // bounded device-side wait gave up.  `stage_polls`: polls of the staging wait before it
@@ -92,6 +95,11 @@ __host__ __device__ inline int edge_bucket(int n) {
     return kEdgeBuckets - 1 - (b < kEdgeBuckets - 1 ? b : kEdgeBuckets - 1);
 }
 
+// A group of lpair: its number, its first sphere and its count (group order).
+__device__ __forceinline__ int pair_group(int w) { return w & 0xff; }
+__device__ __forceinline__ int pair_first(int w) { return (w >> 8) & 0x1ff; }
+__device__ __forceinline__ int pair_count(int w) { return w >> 17; }
+
 constexpr int kMaxGroups = 32;
 constexpr float kBroadMargin = 1e-3f;    // metres added to every group bounding radius
 
@@ -99,17 +107,19 @@ struct DevEnv {
     int ns, nb, nc;
     const float4 *words;              // env_words(ns, nb, nc) float4
     // Distance field of the scene (gbmp_field.cu), or null: field[(iz * ny + iy) * nx + ix]
-    // is the least distance from the centre of cell (ix, iy, iz) to an obstacle; cells of
-    // edge h from the corner (ox, oy, oz); [lo, hi] bounds all obstacles.
-    const float *field;
+    // holds the three least distances from the centre of cell (ix, iy, iz) to an obstacle
+    // and the obstacles of the first two (o1 | o2 << 16 as its bits: spheres 0 .. ns - 1,
+    // then the cuboids, then the cylinders; 0xffff: there is none); cells of edge h from
+    // the corner (ox, oy, oz); [lo, hi] bounds all obstacles.
+    const float4 *field;
     int nx, ny, nz;
     float ox, oy, oz, h, inv_h;
     float lox, loy, loz, hix, hiy, hiz;
 };
 
-// Cells along the field's longest side (128 KB a scene at most).  65,536 edges of the 8-DOF
+// Cells along the field's longest side (512 KB a scene at most).  65,536 edges of the 8-DOF
 // arm in 336 obstacles: 1.255 ms with 32, 1.242 with 48, 1.238 with 64, 1.233 with 128;
-// a scene of 336 obstacles takes 42 us longer to create (72 us; 60 us longer with 48).
+// a scene of 336 obstacles takes 45 us longer to create (76 us; some 60 us longer with 48).
 constexpr int kFieldCells = 32;
 constexpr double kFieldBorder = 0.2;     // metres of field around the obstacles
 constexpr double kFieldLargest = 1.0;    // bounding radius of the obstacles that span the field
@@ -129,7 +139,7 @@ struct SmemTables {
     float4 *grp;
     int *glink, *sgrp;
     int4 *lpair;
-    int *gso, *gsl;
+    int *gso, *place;
     float4 *env;                      // staged environment words
 };
 
@@ -186,7 +196,7 @@ __device__ inline SmemTables carve_tables(unsigned char *base, const DevRobot &R
     t.sgrp = reinterpret_cast<int *>(base + off); off += align16(sizeof(int) * R.S);
     t.lpair = reinterpret_cast<int4 *>(base + off); off += align16(sizeof(int4) * R.NPL);
     t.gso = reinterpret_cast<int *>(base + off); off += align16(sizeof(int) * (R.G + 1));
-    t.gsl = reinterpret_cast<int *>(base + off); off += align16(sizeof(int) * R.S);
+    t.place = reinterpret_cast<int *>(base + off); off += align16(sizeof(int) * R.S);
     t.env = reinterpret_cast<float4 *>(base + off);
     return t;
 }
@@ -294,6 +304,18 @@ __device__ __forceinline__ float mul_elem(const float *A, const float *B, int r,
 __device__ __forceinline__ void rot33(const float *n4, float s, float c, float *R) {
     const float nx = n4[0], ny = n4[1], nz = n4[2], valid = n4[3];
     const float oc = __fadd_rn(1.f, -c);
+    if (valid == 1.f) {   // the axis has a length: the factor 1 and the term 0 below change nothing
+        R[0] = __fmaf_rn(__fmul_rn(nx, nx), oc, c);
+        R[1] = __fmaf_rn(__fmul_rn(nx, ny), oc, -__fmul_rn(nz, s));
+        R[2] = __fmaf_rn(__fmul_rn(nx, nz), oc, __fmul_rn(ny, s));
+        R[3] = __fmaf_rn(__fmul_rn(ny, nx), oc, __fmul_rn(nz, s));
+        R[4] = __fmaf_rn(__fmul_rn(ny, ny), oc, c);
+        R[5] = __fmaf_rn(__fmul_rn(ny, nz), oc, -__fmul_rn(nx, s));
+        R[6] = __fmaf_rn(__fmul_rn(nz, nx), oc, -__fmul_rn(ny, s));
+        R[7] = __fmaf_rn(__fmul_rn(nz, ny), oc, __fmul_rn(nx, s));
+        R[8] = __fmaf_rn(__fmul_rn(nz, nz), oc, c);
+        return;
+    }
     const float iv = __fadd_rn(1.f, -valid);
     R[0] = __fadd_rn(__fmul_rn(__fmaf_rn(__fmul_rn(nx, nx), oc, c), valid), iv);
     R[1] = __fmul_rn(__fmaf_rn(__fmul_rn(nx, ny), oc, -__fmul_rn(nz, s)), valid);
@@ -336,10 +358,7 @@ __device__ __forceinline__ void joint_local_regs(const SmemTables &t, int i, flo
                 acc = __fmaf_rn(P[4 * r + 1], R[3 + c], acc);
                 M[4 * r + c] = __fmaf_rn(P[4 * r + 2], R[6 + c], acc);
             }
-            float acc = __fmul_rn(P[4 * r], 0.f);
-            acc = __fmaf_rn(P[4 * r + 1], 0.f, acc);
-            acc = __fmaf_rn(P[4 * r + 2], 0.f, acc);
-            M[4 * r + 3] = __fadd_rn(acc, P[4 * r + 3]);
+            M[4 * r + 3] = P[4 * r + 3];   // the joint does not translate: its three products are 0
         }
     } else if (ty == 2) {
         const float *a = t.axr + 4 * i;
@@ -412,21 +431,31 @@ __device__ __forceinline__ float sq3(float dx, float dy, float dz) {
 // True when no obstacle of the scene comes within `rad` of (x, y, z): the sphere lies
 // outside the box of all obstacles, or the distance stored for the nearest cell centre,
 // less the way there (distances change by no more than the way), exceeds rad.  False says
-// nothing.  One load (L1 or L2: a field is 128 KB at most) in place of a test
+// nothing.  One load (L1 or L2: a field is 512 KB at most) in place of a test
 // against every obstacle; with the cells of a 2 m scene 6 cm wide the bound is 3 cm short on
 // average.
 // Callers' radii carry kBroadMargin, which covers the rounding here and in the exact tests.
-__device__ __forceinline__ bool scene_far(const DevEnv &E, float x, float y, float z, float rad) {
-    if (!E.field) return E.ns + E.nb + E.nc == 0;
+// Outside the box of all obstacles, by more than rad.
+__device__ __forceinline__ bool scene_outside(const DevEnv &E, float x, float y, float z, float rad) {
     const float ax = fmaxf(fmaxf(E.lox - x, x - E.hix), 0.f), ay = fmaxf(fmaxf(E.loy - y, y - E.hiy), 0.f),
                 az = fmaxf(fmaxf(E.loz - z, z - E.hiz), 0.f);
-    if (ax * ax + ay * ay + az * az > rad * rad) return true;
+    return ax * ax + ay * ay + az * az > rad * rad;
+}
+// The cell nearest to (x, y, z) and the way to its centre.
+__device__ __forceinline__ const float4 *scene_cell(const DevEnv &E, float x, float y, float z, float &way) {
     const int ix = min(max((int)((x - E.ox) * E.inv_h), 0), E.nx - 1), iy = min(max((int)((y - E.oy) * E.inv_h), 0), E.ny - 1),
               iz = min(max((int)((z - E.oz) * E.inv_h), 0), E.nz - 1);
-    const float d = __ldg(E.field + ((iz * E.ny + iy) * E.nx + ix));
     const float dx = x - (E.ox + ((float)ix + 0.5f) * E.h), dy = y - (E.oy + ((float)iy + 0.5f) * E.h),
                 dz = z - (E.oz + ((float)iz + 0.5f) * E.h);
-    return d - sqrtf(dx * dx + dy * dy + dz * dz) > rad;
+    way = sqrtf(dx * dx + dy * dy + dz * dz);
+    return E.field + ((iz * E.ny + iy) * E.nx + ix);
+}
+__device__ __forceinline__ bool scene_far(const DevEnv &E, float x, float y, float z, float rad) {
+    if (!E.field) return E.ns + E.nb + E.nc == 0;
+    if (scene_outside(E, x, y, z, rad)) return true;
+    float way;
+    const float4 *cell = scene_cell(E, x, y, z, way);
+    return __ldg(&cell->x) - way > rad;
 }
 
 // ---------------------------------------------------------------------------------
@@ -753,7 +782,7 @@ __device__ inline bool warp_collide_culled(const SmemTables &t, const DevRobot &
         int p0 = 0, p1 = 0;
         if (k < R.NPL) {
             const int4 lp = t.lpair[k];
-            const float4 a = w.gb[lp.x], b = w.gb[lp.y];
+            const float4 a = w.gb[pair_group(lp.x)], b = w.gb[pair_group(lp.y)];
             const float rr = a.w + b.w;
             on = sq3(a.x - b.x, a.y - b.y, a.z - b.z) < rr * rr;
             p0 = lp.z;
@@ -818,7 +847,7 @@ __device__ inline void store_fk(const SmemTables &t, const DevRobot &R, const Wa
 
 // One state of a collision check, one warp: FK of state s of q, its poses / centres when
 // asked for, the collision test, and the outputs (verdict; in cost mode the four
-// constraint costs [4][n] and their total).  k_check_states and the batched check run
+// constraint costs [4][n] and their total).  k_check_costs and the batched check run
 // this routine, so their outputs are bit-identical.
 template <bool COST, int SPL>
 __device__ inline void check_state(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,

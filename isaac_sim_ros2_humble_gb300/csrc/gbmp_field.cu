@@ -6,24 +6,42 @@
 
 namespace gbmp {
 
-// Least distance of every cell's centre to an obstacle (spheres |c - o| - r, cuboids the
-// distance to the box, cylinders the signed distance): eight lanes a cell, each an eighth
-// of the obstacles (one lane a cell leaves 32,768 threads with a chain over every obstacle:
-// a scene of 336 took 75 us longer to create, 42 us with eight).
+// The three least distances from every cell's centre to an obstacle (spheres |c - o| - r,
+// cuboids the distance to the box, cylinders the signed distance) and the obstacles of the
+// first two: eight lanes a cell, each an eighth of the obstacles, then merged (one lane a
+// cell leaves 32,768 threads with a chain over every obstacle: a scene of 336 took 75 us
+// longer to create, 45 us with eight).
 constexpr int kFieldLanes = 8;
 
-__global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float *__restrict__ field) {
+struct Nearest3 {
+    float d1 = 3.0e38f, d2 = 3.0e38f, d3 = 3.0e38f;
+    int o1 = 0xffff, o2 = 0xffff;
+    __device__ __forceinline__ void add(float d, int o) {
+        if (d >= d3) return;
+        if (d < d2) {
+            d3 = d2;
+            const bool first = d < d1;
+            d2 = first ? d1 : d;
+            o2 = first ? o1 : o;
+            if (first) { d1 = d; o1 = o; }
+        } else {
+            d3 = d;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float4 *__restrict__ field) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, cell = tid / kFieldLanes, o0 = tid % kFieldLanes;
     const bool in = cell < E.nx * E.ny * E.nz;
     const int ix = cell % E.nx, iy = cell / E.nx % E.ny, iz = cell / (E.nx * E.ny);
     const float x = E.ox + ((float)ix + 0.5f) * E.h, y = E.oy + ((float)iy + 0.5f) * E.h,
                 z = E.oz + ((float)iz + 0.5f) * E.h;
-    float best = 3.0e38f;
+    Nearest3 n;
     const float4 *w = E.words;
 #pragma unroll 4
     for (int o = o0; o < E.ns; o += kFieldLanes) {
         const float4 b = __ldg(w + o);
-        best = fminf(best, sqrtf(sq3(x - b.x, y - b.y, z - b.z)) - b.w);
+        n.add(sqrtf(sq3(x - b.x, y - b.y, z - b.z)) - b.w, o);
     }
     w += E.ns;
 #pragma unroll 2
@@ -32,7 +50,7 @@ __global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float *__restrict
         const float3 l = xform_rows(__ldg(w + 5 * o), __ldg(w + 5 * o + 1), __ldg(w + 5 * o + 2), x, y, z);
         const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x), dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y),
                     dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
-        best = fminf(best, sqrtf(sq3(dx, dy, dz)));
+        n.add(sqrtf(sq3(dx, dy, dz)), E.ns + o);
     }
     w += 5 * E.nb;
 #pragma unroll 2
@@ -41,11 +59,18 @@ __global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float *__restrict
         const float3 l = xform_rows(__ldg(w + 4 * o), __ldg(w + 4 * o + 1), __ldg(w + 4 * o + 2), x, y, z);
         const float dx = sqrtf(l.x * l.x + l.y * l.y) - pr.x, dz = fabsf(l.z) - pr.y;
         const float ox = fmaxf(dx, 0.f), oz = fmaxf(dz, 0.f);
-        best = fminf(best, sqrtf(ox * ox + oz * oz) + fminf(fmaxf(dx, dz), 0.f));
+        n.add(sqrtf(ox * ox + oz * oz) + fminf(fmaxf(dx, dz), 0.f), E.ns + E.nb + o);
     }
 #pragma unroll
-    for (int off = 1; off < kFieldLanes; off <<= 1) best = fminf(best, __shfl_xor_sync(kFull, best, off));
-    if (in && o0 == 0) field[cell] = best;
+    for (int off = 1; off < kFieldLanes; off <<= 1) {
+        const float d1 = __shfl_xor_sync(kFull, n.d1, off), d2 = __shfl_xor_sync(kFull, n.d2, off),
+                    d3 = __shfl_xor_sync(kFull, n.d3, off);
+        const int o1 = __shfl_xor_sync(kFull, n.o1, off), o2 = __shfl_xor_sync(kFull, n.o2, off);
+        n.add(d1, o1);
+        n.add(d2, o2);
+        n.add(d3, 0xffff);   // below d1 and d2, so it ends as a third distance at most
+    }
+    if (in && o0 == 0) field[cell] = make_float4(n.d1, n.d2, n.d3, __int_as_float(n.o1 | n.o2 << 16));
 }
 
 // The field's region and cell size from the obstacles' bounding spheres (centre, radius:
@@ -92,7 +117,7 @@ bool scene_field_plan(const std::vector<double> &b, DevEnv &E) {
     return true;
 }
 
-cudaError_t scene_field_build(const DevEnv &E, float *field, cudaStream_t s) {
+cudaError_t scene_field_build(const DevEnv &E, float4 *field, cudaStream_t s) {
     const int cells = E.nx * E.ny * E.nz;
     k_scene_field<<<(cells * kFieldLanes + 255) / 256, 256, 0, s>>>(E, field);
     return cudaGetLastError();

@@ -44,6 +44,9 @@ gbmp_status ensure_smem_optin(const void *fn);
 constexpr int kMaxSelfPairs = 65535 * 4;
 constexpr int kMaxEnvWords = 12 * 1024;     // 192 KB of float4 staged in shared memory
 constexpr int kWarpsPerBlock = 8;
+// dynamic shared memory a block can have next to the staging barrier and flags (227 KB less
+// what ensure_smem_optin leaves to static shared memory)
+constexpr size_t kSmemLimit = 227 * 1024 - 16;
 
 // Growable device buffer owned by a handle.
 struct DevBuf {
@@ -138,6 +141,37 @@ gbmp_status codegen_fk(const gbmp_robot_s *r, const float *q, long long n, float
 gbmp_status codegen_edge_setup(const gbmp_robot_s *r, const float *from, const float *to, long long E, float res,
                                int rule, int *nsteps, float *dir, int *hist, float *length_out, int *nsteps_out,
                                cudaStream_t s);
+// Launch shape of a verdict check: states a warp takes at a time, warps a block, dynamic
+// shared memory, blocks that fit on an SM.  Three blocks of 8 warps an SM at 80 registers:
+// with 64 registers (32 warps) the spills cost more than the warps bring (4,096 states 17.4
+// against 14.4 us).  Up to 7 states at a time: 70,072 states of a 9-DOF arm take 91 us with
+// 3, 79 with 5, 75 with 7 and 84 with 10, whose scratch leaves 16 warps an SM.
+constexpr int kStatesWarps = 8, kStatesResident = 24, kStatesKs = 7;
+struct StatesShape {
+    int ks, warps, per_sm;
+    size_t smem;
+};
+// The shape for a robot and scene whose staged tables take `tables` bytes and whose warps
+// take `bytes(ks)`, with `want` states a warp at most; false when nothing fits.
+template <typename F>
+inline bool states_shape(size_t tables, F bytes, int want, size_t limit, StatesShape *out) {
+    for (int ks = want; ks >= 1; --ks) {
+        StatesShape best{};
+        for (int warps = kStatesWarps; warps >= 1; warps /= 2) {
+            const size_t smem = tables + bytes(ks) * warps;
+            if (smem > limit) continue;
+            // 1 KB a block is the system's, a block's static shared memory some words
+            const int per_sm = (int)std::min<size_t>(kStatesResident / warps, (limit + 2048) / (smem + 2048));
+            if (per_sm * warps > best.per_sm * best.warps) best = StatesShape{ks, warps, per_sm, smem};
+        }
+        if (best.per_sm * best.warps >= 16 || (ks == 1 && best.per_sm)) {
+            *out = best;
+            return true;
+        }
+    }
+    return false;
+}
+
 // How a call's edges are cut into items (gbmp_chunk.cu): parts per edge, the least chunks
 // of a part, and the items a warp takes at a time.  Made on the device by k_edge_order.
 constexpr int kEdgeMaxParts = 64;
@@ -164,7 +198,7 @@ namespace gbmp {
 // Distance field of a scene (gbmp_field.cu): region and cells from the bounding spheres
 // (4 doubles each), then the values, written to `field` on stream s.
 bool scene_field_plan(const std::vector<double> &bounds, DevEnv &E);
-cudaError_t scene_field_build(const DevEnv &E, float *field, cudaStream_t s);
+cudaError_t scene_field_build(const DevEnv &E, float4 *field, cudaStream_t s);
 }  // namespace gbmp
 
 struct gbmp_env_s {

@@ -694,7 +694,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
         GBMP_CHECK_ARG(pr.robot && pr.env && pr.start && pr.goal, "problem %d has a NULL field", i);
         GBMP_CHECK_ARG(pr.robot->L <= b->max_links, "problem %d: %d links > max_links %d", i, pr.robot->L,
                        b->max_links);
-        const DevRobot &R = pr.robot->dev;
+        const DevRobot &R = pr.robot->dev_chunk;   // the edge checks go by chunks
         const DevEnv E = pr.env->dev();
         spl = std::max(spl, R.spl);
         cull = cull && R.cull;
