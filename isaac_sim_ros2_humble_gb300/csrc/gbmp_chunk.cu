@@ -25,7 +25,7 @@ constexpr int kChunkWarps = 8;
 // Why parts: the free edges are few (18 % of the benchmark's) and long, so with one warp
 // per edge most warps idled while some walked up to 56 chunks in a row: 64 edges 0.47 ms
 // whole, 0.046 ms in parts; 3,001 edges of a 30-link robot with first hits 1.20 and 0.30
-// ms; 65,536 edges (18 for each warp) 2.22 and 2.26 ms.
+// ms; 65,536 edges (18 for each warp) 2.22 and 2.26 ms (these with the kernel of that time).
 //
 // The chunk orders are gbmp_order.h's: state order when the first hit is asked for,
 // coarse to fine when only the verdict is.  On the 65,536 edges of the 8-DOF benchmark
@@ -37,11 +37,20 @@ constexpr int kChunkWarps = 8;
 // 65,536 edges, verdicts: 2.22 ms; 3.79 ms when the states were walked one by one, their
 // spheres in the lanes.
 
+// A warp that holds a later part of an edge waits, at most kProbePolls looks, until the
+// edge's probes are known or it has a hit (bits beside the state count).  The warp that holds them took
+// them before this one took its item and does not wait before it has walked them.  Without
+// the wait a batch whose edges collide at once had every part of every edge walked: 161
+// edges 180 us, 54 us with it (63 us with one warp an edge); 64 edges take 40 us
+// with it, 35 without.
+constexpr int kProbed0 = 1 << 28, kProbed1 = 1 << 29, kHit = 1 << 30, kStepsMask = kProbed0 - 1;
+constexpr int kProbePolls = 4096;
+constexpr int kMaxGrab = 8;   // settled items taken at a time in a batch of few edges
+
 template <int K, bool CNT>
 __global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     k_edge_chunk(DevRobot R, DevEnv E, const float *__restrict__ from, const float *__restrict__ to,
-                 const int *__restrict__ nsteps, const float *__restrict__ dir, const int *__restrict__ order,
-                 int n_edges, const EdgePlan *__restrict__ plan, unsigned long long *__restrict__ next,
+                 int *nsteps, const float *__restrict__ dir, const int *__restrict__ order, int n_edges, const EdgePlan *__restrict__ plan, unsigned long long *__restrict__ next,
                  unsigned char *ok_out, int *first_hit_out) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nwords = env_words(E.ns, E.nb, E.nc);
@@ -52,49 +61,84 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     carve_chunk(smem + smem_tables_bytes(R, nwords), R, K, warp, cs);
     const int lane = threadIdx.x & 31;
     const bool any = first_hit_out == nullptr;
-    const int parts = plan->parts, span0 = plan->span, grab = plan->grab;
-    const long long items = (long long)n_edges * parts;
-    // the other warps' findings (relaxed reads: a late look costs a chunk, not the result)
-    auto settled = [&](int e, int first_state) {
-        return any ? ok_out && *(volatile unsigned char *)(ok_out + e) == 0
-                   : *(volatile unsigned *)(first_hit_out + e) <= (unsigned)first_state;
-    };
+    // What is needed between chunks only lives in shared memory: the chunk routine takes
+    // every register (80, three blocks an SM).
+    __shared__ EdgePlan s_plan;
+    __shared__ int4 s_item[kChunkWarps][kWarp];   // edge, states, first chunk, end
+    if (threadIdx.x == 0) s_plan = *plan;
+    __syncthreads();
+    int grab = s_plan.grab;
     for (;;) {
-        unsigned long long i0 = 0;
-        if (lane == 0) i0 = atomicAdd(next, (unsigned long long)grab);
-        i0 = __shfl_sync(kFull, i0, 0);
-        if ((long long)i0 >= items) break;
-        const long long i = (long long)i0 + lane;
-        int e = 0, n = 0, c0 = 0, c1 = 0;
-        if (lane < grab && i < items) {
-            const int p = (int)(i / n_edges);
-            e = order[i - (long long)p * n_edges];
-            n = nsteps[e];
-            if (n <= kMaxEdgeStates) {
-                const int nch = edge_chunk_count(n, K, any);
-                const int span = max(span0, (nch + parts - 1) / parts);
-                c0 = p * span;
-                c1 = min(c0 + span, nch);
-                if (p > 0 && c0 < c1 && settled(e, edge_chunk_range(c0, n, K, any).x)) c1 = c0;
-            }
-        }
-        for (unsigned live = __ballot_sync(kFull, c0 < c1); live; live &= live - 1u) {
-            const int x = __ffs(live) - 1;
-            const int we = __shfl_sync(kFull, e, x), wn = __shfl_sync(kFull, n, x);
-            const int wc0 = __shfl_sync(kFull, c0, x), wc1 = __shfl_sync(kFull, c1, x);
-            const long long off = (long long)we * R.L;
-            for (int c = wc0; c < wc1; ++c) {
-                const StateRange r = edge_chunk_range(c, wn, K, any);
-                if (parts > 1 && c > wc0 && __any_sync(kFull, settled(we, r.x))) break;
-                const int h = warp_edge_chunk<K, CNT>(t, R, E, cs, lane, from + off, to + off, dir + off, r.x, r.y, wn,
-                                                      any);
-                if (h >= 0) {
-                    if (lane == 0) {
-                        if (ok_out) *(volatile unsigned char *)(ok_out + we) = 0;
-                        if (first_hit_out) atomicMin(reinterpret_cast<unsigned *>(first_hit_out + we), (unsigned)h);
-                    }
-                    break;
+        unsigned live;
+        {
+            const int parts = s_plan.parts;
+            unsigned long long i0 = 0;
+            if (lane == 0) i0 = atomicAdd(next, (unsigned long long)grab);
+            i0 = __shfl_sync(kFull, i0, 0);
+            const long long items = (long long)n_edges * parts, i = (long long)i0 + lane;
+            if ((long long)i0 >= items) break;
+            bool mine = false;
+            if (lane < grab && i < items) {
+                const int p = (int)(i / n_edges);
+                const int e = order[i - (long long)p * n_edges];
+                const int v = *(volatile int *)(nsteps + e), n = v & kStepsMask;
+                if (n <= kMaxEdgeStates && !(any && (v & kHit))) {
+                    const int nch = edge_chunk_count(n, K, any);
+                    const int span = max(s_plan.span, (nch + parts - 1) / parts);
+                    const int c0 = p * span, c1 = min(c0 + span, nch);
+                    mine = c0 < c1 && (any || p == 0 ||
+                                       *(volatile unsigned *)(first_hit_out + e) > (unsigned)edge_chunk_range(c0, n, K, any).x);
+                    s_item[warp][lane] = make_int4(e, n, c0, c1);
                 }
+            }
+            live = __ballot_sync(kFull, mine);   // also orders the items before their reads
+            __syncwarp();
+            // settled items go faster and faster in a batch of few edges
+            grab = live || !s_plan.grow ? s_plan.grab : min(2 * grab, kMaxGrab);
+        }
+        for (; live; live &= live - 1u) {
+            const int x = __ffs(live) - 1;
+            if (s_plan.probing) {
+                const int4 it = s_item[warp][x];
+                // the probes (the first chunk, and for verdicts the last) come first: an edge
+                // they settle is not walked by the warps that hold its other parts
+                const int probes = any ? min(2, edge_chunk_count(it.y, K, any)) : 1;
+                if (it.z >= probes) {
+                    const int want = probes == 2 ? kProbed0 | kProbed1 : kProbed0;
+                    bool hit = false;
+                    for (int poll = 0; poll < kProbePolls; ++poll) {
+                        const int v = *(volatile int *)(nsteps + it.x);
+                        hit = any ? (v & kHit) != 0
+                                  : *(volatile unsigned *)(first_hit_out + it.x) <= (unsigned)edge_chunk_range(it.z, it.y, K, any).x;
+                        if (__any_sync(kFull, (v & want) == want || hit)) break;
+                        __nanosleep(200);
+                    }
+                    if (__any_sync(kFull, hit)) continue;
+                }
+            }
+            for (int c = s_item[warp][x].z;; ++c) {
+                const int4 it = s_item[warp][x];
+                if (c >= it.w) break;
+                const StateRange r = edge_chunk_range(c, it.y, K, any);
+                // the other warps' findings (relaxed: a late look costs a chunk, not the result)
+                if (c > it.z) {
+                    const bool settled = any ? (*(volatile int *)(nsteps + it.x) & kHit) != 0
+                                             : *(volatile unsigned *)(first_hit_out + it.x) <= (unsigned)r.x;
+                    if (__any_sync(kFull, settled)) break;
+                }
+                const long long off = (long long)it.x * R.L;
+                const int h = warp_edge_chunk<K, CNT>(t, R, E, cs, lane, from + off, to + off, dir + off, r.x, r.y,
+                                                      it.y, any);
+                const int e = s_item[warp][x].x;
+                if (lane == 0) {
+                    if (h >= 0) {
+                        if (ok_out) *(volatile unsigned char *)(ok_out + e) = 0;
+                        if (first_hit_out) atomicMin(reinterpret_cast<unsigned *>(first_hit_out + e), (unsigned)h);
+                    }
+                    if (h >= 0 || (s_plan.probing && c < 2))
+                        atomicOr(nsteps + e, (h >= 0 ? kHit : 0) | (c == 0 ? kProbed0 : c == 1 ? kProbed1 : 0));
+                }
+                if (h >= 0) break;
             }
         }
         __syncwarp();
@@ -134,7 +178,7 @@ gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, 
 int edge_chunk_warps(int grid) { return grid * kChunkWarps; }
 
 gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int grid, size_t smem, cudaStream_t s,
-                              const float *from, const float *to, const int *nsteps, const float *dir,
+                              const float *from, const float *to, int *nsteps, const float *dir,
                               const int *order, long long n_edges, const EdgePlan *plan, unsigned long long *next,
                               unsigned char *ok, int *first_hit) {
     // the grid is the resident blocks, at most one warp per item
@@ -181,7 +225,7 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
         const long long s0 = c * kFkChunk;
         const int ks = (int)min((long long)kFkChunk, n - s0);
         const float *qc = q + s0 * L;
-        warp_fk_chunk_q<kFkChunk>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, lpK, lane);
+        warp_fk_chunk_q<kFkChunk, 4>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, lpK, lane);
         store_fk_states(t, L, S, lpK, s0, ks, poses, centers, vec, lane);
         __syncwarp();
     }

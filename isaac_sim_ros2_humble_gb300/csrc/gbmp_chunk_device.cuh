@@ -30,7 +30,9 @@
 // against every run, 1.25 ms with the field (most chunks then have no group left).  Walking the states one after another left most lanes idle: per state of the
 // benchmark's edges 0.3 obstacle candidates and 2.3 group pairs, each pair's test a chain
 // of shared-memory loads over 7 spheres.  Side by side the chunk's 23 (state, pair) items
-// fill a warp.
+// fill a warp.  And the size of the code counts: the chunk kernel's loops are not unrolled
+// (51 KB instead of 75 KB; 65,536 edges 1.21 against 1.25 ms), for the instruction cache
+// holds about one such body.
 #pragma once
 
 #include "gbmp_internal.h"
@@ -68,9 +70,10 @@ __device__ inline void carve_chunk(unsigned char *base, const DevRobot &R, int K
 // identity and needs none), then the chains, one pose row a lane (below), each pose
 // written over the joint-local transform it is made from.  qv(k, i) is joint i of state
 // k.  The arithmetic is warp_fk's (joint_local, mul_elem), so poses are bit-identical.
-template <int K, typename QV>
+template <int K, int UNROLL = 1, typename QV>
 __device__ inline void warp_fk_chunk_q(const SmemTables &t, int L, int ks, QV qv, float *lpK, int lane) {
     const unsigned rks = (65536u + ks - 1u) / ks;   // idx / ks = idx * rks >> 16 (idx < 64 * 10)
+#pragma unroll UNROLL
     for (int idx = lane; idx < ks * (L - 1); idx += kWarp) {
         const int i = 1 + (int)(idx * rks >> 16), k = idx - (i - 1) * ks;
         joint_local(t, i, qv(k, i), lpK + 12 * (k * L + i));
@@ -90,6 +93,7 @@ __device__ inline void warp_fk_chunk_q(const SmemTables &t, int L, int ks, QV qv
     const float4 unit = make_float4(rr == 0 ? 1.f : 0.f, rr == 1 ? 1.f : 0.f, rr == 2 ? 1.f : 0.f, 0.f);
     float4 a = unit;
     if (own) *rowp = a;
+#pragma unroll UNROLL
     for (int i = 1; i < L; ++i) {
         const int ty = t.type[i], par = t.parent[i];
         float4 o = unit;
@@ -133,6 +137,7 @@ __device__ __forceinline__ unsigned run_groups(const float4 *runs, int nruns, in
     unsigned gm = 0u;
     if (c < nruns) {
         const float4 b = runs[c];
+#pragma unroll 1
         for (unsigned m = groups; m; m &= m - 1u) {
             const int q = __ffs(m) - 1;
             const float4 gs = cs.sgb[q];
@@ -190,11 +195,13 @@ __device__ __forceinline__ int chunk_obstacle(const SmemTables &t, const DevRobo
         r0 = cy[0]; r1 = cy[1]; r2 = cy[2]; p3 = cy[3];
     }
     int hk = kmax;
+#pragma unroll 1
     for (; gm; gm &= gm - 1u) {
         const int g = __ffs(gm) - 1;
         const int g0 = t.gso[g], ng = t.gso[g + 1] - g0, total = ng * kmax;
         const float *T = lpK + 12 * t.glink[g];
         const float inv = 1.f / (float)ng;
+#pragma unroll 1
         for (int idx = lane; idx < total; idx += kWarp) {
             const int k = (int)(((float)idx + 0.5f) * inv);   // idx / ng (idx < 2^12)
             float4 s;
@@ -244,6 +251,7 @@ __device__ __forceinline__ bool group_pair_hits(const SmemTables &t, const DevRo
     const bool full = pr.w - pr.z == na * nb;
     const float *TA = lp + 12 * t.glink[pair_group(pr.x)], *TB = lp + 12 * t.glink[pair_group(pr.y)];
     const int nbw = __reduce_max_sync(kFull, full ? nb : 0);
+#pragma unroll 1
     for (int jb = 0; jb < nbw; jb += 8) {
         bool ib = false;
         if (full && jb + sl < nb) {
@@ -254,11 +262,13 @@ __device__ __forceinline__ bool group_pair_hits(const SmemTables &t, const DevRo
         }
         const unsigned mb = (__ballot_sync(kFull, ib) >> sh) & 0xffu;
         if (mb) {
+#pragma unroll 1
             for (int ja = sl; ja < na; ja += 8) {
                 float4 s;
                 const float3 c = sphere_centre(t, TA, pair_first(pr.x) + ja, s);
                 const float rr = s.w + GB.w;
                 if (sq3(c.x - GB.x, c.y - GB.y, c.z - GB.z) < rr * rr) {
+#pragma unroll 1
                     for (unsigned m = mb; m; m &= m - 1u) {
                         float4 sb;
                         const float3 cb = sphere_centre(t, TB, b0 + jb + __ffs(m) - 1, sb);
@@ -274,6 +284,7 @@ __device__ __forceinline__ bool group_pair_hits(const SmemTables &t, const DevRo
         }
     }
     if (!full)
+#pragma unroll 1
         for (int p = pr.z + sl; p < pr.w; p += 8) {
             const unsigned ij = __ldg(R.pairs + p);
             const float thr = __ldg(R.thr + p);
@@ -296,6 +307,7 @@ __device__ __forceinline__ int chunk_self(const SmemTables &t, const DevRobot &R
     const float inv = 1.f / (float)npr;
     const int sub = lane >> 3, sl = lane & 7, sh = lane & 24;
     int hk = kmax;
+#pragma unroll 1
     for (int i0 = 0; i0 < total; i0 += kWarp) {
         const int idx = i0 + lane;
         bool on = false;
@@ -315,6 +327,7 @@ __device__ __forceinline__ int chunk_self(const SmemTables &t, const DevRobot &R
         if (on) cs.it[__popc(bal & ((1u << lane) - 1u))] = item;
         __syncwarp();
         const int nit = __popc(bal);
+#pragma unroll 1
         for (int j0 = 0; j0 < nit; j0 += 4) {
             int k = 0;
             int4 pr = make_int4(0, 0, 0, 0);
@@ -358,12 +371,14 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
         const float4 g = t.grp[gq];
         const float *T = cs.lpK + 12 * t.glink[gq];
         gr = g.w;
+#pragma unroll 1
         for (int k = lane / gw; k < ks; k += kWarp / gw) {
             const float3 c = xform_point_a16(T + k * 12 * R.L, g.x, g.y, g.z);
             lox = fminf(lox, c.x); loy = fminf(loy, c.y); loz = fminf(loz, c.z);
             hix = fmaxf(hix, c.x); hiy = fmaxf(hiy, c.y); hiz = fmaxf(hiz, c.z);
         }
     }
+#pragma unroll 1
     for (int off = gw; off < kWarp; off <<= 1) {
         lox = fminf(lox, __shfl_xor_sync(kFull, lox, off));
         loy = fminf(loy, __shfl_xor_sync(kFull, loy, off));
@@ -422,6 +437,7 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
                 if (o < E.ns) {
                     const float4 b = sx[o];
                     const float nb = snb[o];
+#pragma unroll 1
                     for (unsigned m = gm; m; m &= m - 1u) {
                         const int q = __ffs(m) - 1;
                         const float4 gs = cs.sgb[q];
@@ -434,6 +450,7 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
                 const int o = (c - nrs) * kWarp + lane;
                 if (o < E.nb) {
                     const float4 r0 = bx[5 * o], r1 = bx[5 * o + 1], r2 = bx[5 * o + 2], mn = bx[5 * o + 3], mx = bx[5 * o + 4];
+#pragma unroll 1
                     for (unsigned m = gm; m; m &= m - 1u) {
                         const int q = __ffs(m) - 1;
                         const float4 gs = cs.sgb[q];
@@ -449,6 +466,7 @@ __device__ inline int warp_edge_chunk(const SmemTables &t, const DevRobot &R, co
                 const int o = (c - nrs - nrb) * kWarp + lane;
                 if (o < E.nc) {
                     const float4 r0 = cyl[4 * o], r1 = cyl[4 * o + 1], r2 = cyl[4 * o + 2], pr = cyl[4 * o + 3];
+#pragma unroll 1
                     for (unsigned m = gm; m; m &= m - 1u) {
                         const int q = __ffs(m) - 1;
                         const float4 gs = cs.sgb[q];

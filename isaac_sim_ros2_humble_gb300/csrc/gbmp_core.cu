@@ -196,7 +196,7 @@ __global__ void k_edge_order(const int *__restrict__ nsteps, long long E, const 
                 const int span = max(1, min(kMaxSpan, (int)(chunks / (4.f * kItemsPerWarp * warps))));
                 const int parts = max(1, min(kEdgeMaxParts, (most + span - 1) / span));
                 const int grab = (int)max(1LL, min(32LL, E * parts / ((long long)kGrabsPerWarp * warps)));
-                *plan = EdgePlan{parts, span, grab, 0};
+                *plan = EdgePlan{parts, span, grab, parts > 1 && E < warps, E < 2 * warps};
             }
         }
     }

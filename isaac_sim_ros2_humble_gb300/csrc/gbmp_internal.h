@@ -173,10 +173,12 @@ inline bool states_shape(size_t tables, F bytes, int want, size_t limit, StatesS
 }
 
 // How a call's edges are cut into items (gbmp_chunk.cu): parts per edge, the least chunks
-// of a part, and the items a warp takes at a time.  Made on the device by k_edge_order.
+// of a part, the items a warp takes at a time, whether the probes come first (fewer edges
+// than warps: later parts would start at once) and whether settled items go ever faster.
+// Made on the device by k_edge_order.
 constexpr int kEdgeMaxParts = 64;
 struct EdgePlan {
-    int parts, span, grab, pad;
+    int parts, span, grab, probing, grow;
 };
 // Warps of the chunk kernel resident in `grid` blocks.
 int edge_chunk_warps(int grid);
@@ -189,7 +191,7 @@ gbmp_status fk_chunk_launch(const DevRobot &R, int num_sms, const float *q, long
                             float *centers, cudaStream_t s);
 gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, int K, size_t *smem, int *grid);
 gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int grid, size_t smem, cudaStream_t s,
-                              const float *from, const float *to, const int *nsteps, const float *dir,
+                              const float *from, const float *to, int *nsteps, const float *dir,
                               const int *order, long long n_edges, const EdgePlan *plan, unsigned long long *next,
                               unsigned char *ok, int *first_hit);
 }  // namespace gbmp

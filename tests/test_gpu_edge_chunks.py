@@ -98,3 +98,25 @@ def test_outputs_of_long_and_free_edges_without_any_hit():
     np.testing.assert_array_equal(ok, [1, 0, 1, 1, 1])
     np.testing.assert_array_equal(fh, [-1, -2, -1, -1, -1])
     np.testing.assert_array_equal(_run(R, E, a, b, 2e-7, False)[0], ok)
+
+
+@pytest.mark.parametrize("n", [3, 160, 700, 5000])
+def test_batches_whose_edges_are_settled_by_their_probes(n):
+    """Every edge starts, or ends, in collision, or only some do: later parts are dropped."""
+    robot = W.serial_arm(58, dof=7, n_spheres=50)
+    env = W.random_env(59, 60, 10, 4, oriented=True)
+    R, E = api.Robot(robot), api.Env(env)
+    q = torch.from_numpy(robot.sample_full(np.random.default_rng(n), 30000)).cuda()
+    v = torch.zeros(30000, dtype=torch.uint8, device="cuda")
+    api.check_states(R, E, q, v)
+    hit, free = q[v == 1], q[v == 0]
+    for a, b in ((hit[:n], free[:n]), (free[:n], hit[:n]), (torch.cat([hit[: n // 2], free[: n - n // 2]]), free[n: 2 * n])):
+        a, b = a.contiguous(), b.contiguous()
+        R.set_edge_form(1)
+        want = _run(R, E, a, b, 0.01, True)
+        R.set_edge_form(0)
+        for k in range(3):
+            got = _run(R, E, a, b, 0.01, True)
+            np.testing.assert_array_equal(got[0], want[0])
+            np.testing.assert_array_equal(got[1], want[1])
+            np.testing.assert_array_equal(_run(R, E, a, b, 0.01, False)[0], want[0])
