@@ -6,7 +6,7 @@
 // outputs), and a second table splits their states into block-sized ranges; every block
 // stages the tables of its own request into shared memory (bulk asynchronous copies) and
 // checks its range with the routines of k_check_verdicts (several states a warp,
-// check_verdicts) or k_check_costs (one, check_state), so each request's outputs are
+// check_verdicts) or k_check_costs (one, check_costs), so each request's outputs are
 // bit-identical to a gbmp_check_states_fk call of its own.  Shared memory is sized for the
 // largest request; the spheres-per-lane template of the costs covers the robot with the
 // most spheres (smaller robots leave slots empty).
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (long long s = sB.lo + threadIdx.x / kWarp; s < sB.hi; s += kWarpsPerBlock)
-        check_state<true, SPL>(t, R, E, w, sT.q, s, sT.n, sT.verdict, sT.costs, sT.total, sT.poses, sT.centers, lane);
+        check_costs<SPL>(t, R, E, w, sT.q, s, sT.n, sT.verdict, sT.costs, sT.total, sT.poses, sT.centers, lane);
 }
 
 // `ks` states a warp at a time.  256 requests over 4 robots and 16 scenes, 1.57 million

@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     }
 }
 
-// Costs of n states; one warp per state.  With poses / centers non-null the FK of each
-// state is also written out (the reference's update() and checkStates() from one FK).
+// Costs of n states; one warp per state (warp_costs).  With poses / centers non-null the FK of
+// each state is also written out (the reference's update() and checkStates() from one FK).
 template <int SPL>
 __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
     k_check_costs(DevRobot R, DevEnv E, const float *__restrict__ q, long long n, unsigned char *__restrict__ verdict,
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
     const int lane = threadIdx.x & 31;
     const long long nw = (long long)gridDim.x * kWarpsPerBlock;
     for (long long s = blockIdx.x * (long long)kWarpsPerBlock + threadIdx.x / kWarp; s < n; s += nw)
-        check_state<true, SPL>(t, R, E, w, q, s, n, verdict, costs, total, poses, centers, lane);
+        check_costs<SPL>(t, R, E, w, q, s, n, verdict, costs, total, poses, centers, lane);
 }
 
 // Collision verdicts of n states, `ks` states a warp at a time (gbmp_states_device.cuh).
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, CULL ? 3 : 1)
                 __syncwarp();
                 warp_fk(t, R.L, w, lane);
                 const bool h = CULL ? warp_collide_culled<SPL>(t, R, E, w, lane)
-                                    : warp_collide<SPL, false>(t, R, E, w, lane, nullptr);
+                                    : warp_collide<SPL>(t, R, E, w, lane);
                 __syncwarp();
                 if (h) { hit = s; break; }
             }

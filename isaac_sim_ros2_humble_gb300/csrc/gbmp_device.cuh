@@ -459,15 +459,11 @@ __device__ __forceinline__ bool scene_far(const DevEnv &E, float x, float y, flo
 }
 
 // ---------------------------------------------------------------------------------
-// Collision of one state.  Returns true if it collides.  With COST, costs[0..3] of
-// lane 0 receive the warp totals per constraint slot (self, spheres, cuboids,
-// cylinders), following the per-pair cost formulas of SelfCollisionConstraint.cu:80-112,
-// EnvConstraintSphere.cu:57-96, EnvConstraintCuboid.cu:105-159,
-// EnvConstraintCylinder.cu:130-180.
+// Collision of one state.  Returns true if it collides.
 // ---------------------------------------------------------------------------------
-template <int SPL, bool COST>
+template <int SPL>
 __device__ inline bool warp_collide(const SmemTables &t, const DevRobot &R, const DevEnv &E,
-                                    const WarpScratch &w, int lane, float *costs) {
+                                    const WarpScratch &w, int lane) {
     float cx[SPL], cy[SPL], cz[SPL], cr[SPL];
 #pragma unroll
     for (int m = 0; m < SPL; ++m) {
@@ -484,44 +480,31 @@ __device__ inline bool warp_collide(const SmemTables &t, const DevRobot &R, cons
     __syncwarp();
 
     bool hit = false;
-    float c_self = 0.f, c_sph = 0.f, c_box = 0.f, c_cyl = 0.f;
     const float4 *env = t.env;
 
     // --- environment spheres ---
-    if (COST) {
-        for (int o = 0; o < E.ns; ++o) {
-            const float4 b = env[o];
+    // Expanded form: d^2 - (rs + ro)^2 = A + B - 2 (c.o + rs ro) with A = |c|^2 - rs^2
+    // per robot sphere and B = |o|^2 - ro^2 per obstacle (staged as (2o, 2ro, -B)),
+    // so a test is four FMAs and a compare.  Rounding moves the contact surface by
+    // ~1e-5 m at workspace scale.
+    float A[SPL];
+#pragma unroll
+    for (int m = 0; m < SPL; ++m) A[m] = __fmaf_rn(cz[m], cz[m], __fmaf_rn(cy[m], cy[m], __fmaf_rn(cx[m], cx[m], -cr[m] * cr[m])));
+    const float4 *sx = t.env + E.ns + 5 * E.nb + 4 * E.nc;
+    const float *snb = reinterpret_cast<const float *>(sx + E.ns);
+    for (int o0 = 0; o0 < E.ns; o0 += 16) {
+        const int oe = min(o0 + 16, E.ns);
+#pragma unroll 4
+        for (int o = o0; o < oe; ++o) {
+            const float4 b = sx[o];
+            const float nb = snb[o];
 #pragma unroll
             for (int m = 0; m < SPL; ++m) {
-                const float d2 = sq3(cx[m] - b.x, cy[m] - b.y, cz[m] - b.z);
-                const float rr = cr[m] + b.w;
-                if (d2 < rr * rr) c_sph += fmaxf(0.f, rr - sqrtf(d2));
+                const float v = __fmaf_rn(cx[m], b.x, __fmaf_rn(cy[m], b.y, __fmaf_rn(cz[m], b.z, __fmaf_rn(cr[m], b.w, nb))));
+                hit |= v > A[m];
             }
         }
-    } else {
-        // Expanded form: d^2 - (rs + ro)^2 = A + B - 2 (c.o + rs ro) with A = |c|^2 - rs^2
-        // per robot sphere and B = |o|^2 - ro^2 per obstacle (staged as (2o, 2ro, -B)),
-        // so a test is four FMAs and a compare.  Rounding moves the contact surface by
-        // ~1e-5 m at workspace scale.
-        float A[SPL];
-#pragma unroll
-        for (int m = 0; m < SPL; ++m) A[m] = __fmaf_rn(cz[m], cz[m], __fmaf_rn(cy[m], cy[m], __fmaf_rn(cx[m], cx[m], -cr[m] * cr[m])));
-        const float4 *sx = t.env + E.ns + 5 * E.nb + 4 * E.nc;
-        const float *snb = reinterpret_cast<const float *>(sx + E.ns);
-        for (int o0 = 0; o0 < E.ns; o0 += 16) {
-            const int oe = min(o0 + 16, E.ns);
-#pragma unroll 4
-            for (int o = o0; o < oe; ++o) {
-                const float4 b = sx[o];
-                const float nb = snb[o];
-#pragma unroll
-                for (int m = 0; m < SPL; ++m) {
-                    const float v = __fmaf_rn(cx[m], b.x, __fmaf_rn(cy[m], b.y, __fmaf_rn(cz[m], b.z, __fmaf_rn(cr[m], b.w, nb))));
-                    hit |= v > A[m];
-                }
-            }
-            if (__any_sync(kFull, hit)) return true;
-        }
+        if (__any_sync(kFull, hit)) return true;
     }
     env += E.ns;
 
@@ -537,13 +520,10 @@ __device__ inline bool warp_collide(const SmemTables &t, const DevRobot &R, cons
                 const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x);
                 const float dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y);
                 const float dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
-                const float d2 = sq3(dx, dy, dz);
-                const bool h = d2 < cr[m] * cr[m];
-                if (COST) { if (h) c_box += cr[m] - sqrtf(d2); }
-                hit |= h;
+                hit |= sq3(dx, dy, dz) < cr[m] * cr[m];
             }
         }
-        if (!COST && __any_sync(kFull, hit)) return true;
+        if (__any_sync(kFull, hit)) return true;
     }
     env += 5 * E.nb;
 
@@ -562,11 +542,10 @@ __device__ inline bool warp_collide(const SmemTables &t, const DevRobot &R, cons
                 const float outside = sqrtf(__fmaf_rn(oz, oz, __fmul_rn(ox, ox)));
                 const float inside = fminf(fmaxf(dx, dz), 0.f);
                 const float pen = cr[m] - (outside + inside);
-                if (COST) c_cyl += pen > 0.f ? pen : 0.f;
                 hit |= pen > 0.f;
             }
         }
-        if (!COST && __any_sync(kFull, hit)) return true;
+        if (__any_sync(kFull, hit)) return true;
     }
 
     // --- self collision pairs ---
@@ -578,25 +557,12 @@ __device__ inline bool warp_collide(const SmemTables &t, const DevRobot &R, cons
                 const unsigned ij = __ldg(R.pairs + p);
                 const float thr = __ldg(R.thr + p);
                 const float4 a = w.cen[ij & 0xffffu], b = w.cen[ij >> 16];
-                const float d2 = sq3(a.x - b.x, a.y - b.y, a.z - b.z);
-                const bool h = d2 < thr;
-                if (COST) { if (h) c_self += sqrtf(thr) - sqrtf(d2); }
-                hit |= h;
+                hit |= sq3(a.x - b.x, a.y - b.y, a.z - b.z) < thr;
             }
         }
-        if (!COST && __any_sync(kFull, hit)) return true;
+        if (__any_sync(kFull, hit)) return true;
     }
 
-    if (COST) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            c_self += __shfl_xor_sync(kFull, c_self, off);
-            c_sph += __shfl_xor_sync(kFull, c_sph, off);
-            c_box += __shfl_xor_sync(kFull, c_box, off);
-            c_cyl += __shfl_xor_sync(kFull, c_cyl, off);
-        }
-        costs[0] = c_self; costs[1] = c_sph; costs[2] = c_box; costs[3] = c_cyl;
-    }
     return __any_sync(kFull, hit);
 }
 
@@ -808,20 +774,155 @@ __device__ inline bool warp_collide_culled(const SmemTables &t, const DevRobot &
 #undef GBMP_CULLED_RETURN
 }
 
-// Dispatch on spheres-per-lane.
-template <bool COST>
-__device__ inline bool warp_collide_dispatch(const SmemTables &t, const DevRobot &R, const DevEnv &E,
-                                             const WarpScratch &w, int lane, float *costs) {
-    switch (R.spl) {
-    case 1: return warp_collide<1, COST>(t, R, E, w, lane, costs);
-    case 2: return warp_collide<2, COST>(t, R, E, w, lane, costs);
-    case 3: return warp_collide<3, COST>(t, R, E, w, lane, costs);
-    case 4: return warp_collide<4, COST>(t, R, E, w, lane, costs);
-    case 5: return warp_collide<5, COST>(t, R, E, w, lane, costs);
-    case 6: return warp_collide<6, COST>(t, R, E, w, lane, costs);
-    case 7: return warp_collide<7, COST>(t, R, E, w, lane, costs);
-    default: return warp_collide<8, COST>(t, R, E, w, lane, costs);
+// Costs of one state per constraint slot (self, spheres, cuboids, cylinders), costs[0..3] on
+// every lane: the per-pair formulas of SelfCollisionConstraint.cu:80-112,
+// EnvConstraintSphere.cu:57-96, EnvConstraintCuboid.cu:105-159,
+// EnvConstraintCylinder.cu:130-180, summed over the pairs that can touch.  A sphere that the
+// scene's field clears takes part in no scene term, nor does a run of 32 obstacles that no
+// sphere left reaches; self pairs go by group pairs whose spheres overlap.  What is passed
+// over adds nothing: every term of it is 0.  Summing all pairs (336 obstacles x 110 spheres
+// and 3,192 self pairs a state) took 628 us for 20,011 states, 222 us now.
+template <int SPL>
+__device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
+                                  int lane, float *costs) {
+    float cx[SPL], cy[SPL], cz[SPL], cr[SPL];
+    unsigned left = 0u;   // bit m: some lane's sphere m is left
+#pragma unroll
+    for (int m = 0; m < SPL; ++m) {
+        const int k = lane + kWarp * m;
+        cx[m] = kFar; cy[m] = kFar; cz[m] = kFar; cr[m] = 0.f;
+        bool near = false;
+        if (k < R.S) {
+            const float4 s = t.sph[k];
+            const float3 p = xform_point(w.lp + 12 * t.slink[k], s.x, s.y, s.z);
+            w.cen[k] = make_float4(p.x, p.y, p.z, s.w);
+            near = !scene_far(E, p.x, p.y, p.z, s.w + kBroadMargin);
+            if (near) { cx[m] = p.x; cy[m] = p.y; cz[m] = p.z; cr[m] = s.w; }
+        }
+        left |= __any_sync(kFull, near) ? 1u << m : 0u;
     }
+    for (int g = lane; g < R.G; g += kWarp) {
+        const float4 s = t.grp[g];
+        const float3 c = xform_point(w.lp + 12 * t.glink[g], s.x, s.y, s.z);
+        w.gb[g] = make_float4(c.x, c.y, c.z, s.w);
+    }
+    __syncwarp();
+
+    float c_self = 0.f, c_sph = 0.f, c_box = 0.f, c_cyl = 0.f;
+    const float4 *runs = t.env + env_cluster_base(E.ns, E.nb, E.nc);
+    // whether some sphere left reaches run i
+    auto reached = [&](int i) {
+        const float4 b = runs[i];
+        bool on = false;
+#pragma unroll
+        for (int m = 0; m < SPL; ++m) {
+            const float rr = cr[m] + kBroadMargin + b.w;
+            on |= !(sq3(cx[m] - b.x, cy[m] - b.y, cz[m] - b.z) >= rr * rr);   // NaN: as the terms have it
+        }
+        return __any_sync(kFull, on) != 0;
+    };
+    if (left) {
+        // --- environment spheres ---
+        const int nrs = env_clusters(E.ns), nrb = env_clusters(E.nb), nrc = env_clusters(E.nc);
+#pragma unroll 1
+        for (int i = 0; i < nrs; ++i) {
+            if (!reached(i)) continue;
+            const int end = min(E.ns, (i + 1) * kWarp);
+#pragma unroll 2
+            for (int o = i * kWarp; o < end; ++o) {
+                const float4 b = t.env[o];
+#pragma unroll
+                for (int m = 0; m < SPL; ++m) {
+                    if (!(left >> m & 1u)) continue;
+                    const float d2 = sq3(cx[m] - b.x, cy[m] - b.y, cz[m] - b.z);
+                    const float rr = cr[m] + b.w;
+                    if (d2 < rr * rr) c_sph += fmaxf(0.f, rr - sqrtf(d2));
+                }
+            }
+        }
+        // --- cuboids (inverse pose, clamp to [min, max]) ---
+        const float4 *bx = t.env + E.ns;
+#pragma unroll 1
+        for (int i = 0; i < nrb; ++i) {
+            if (!reached(nrs + i)) continue;
+            const int end = min(E.nb, (i + 1) * kWarp);
+#pragma unroll 1
+            for (int o = i * kWarp; o < end; ++o) {
+                const float4 r0 = bx[5 * o], r1 = bx[5 * o + 1], r2 = bx[5 * o + 2], mn = bx[5 * o + 3], mx = bx[5 * o + 4];
+#pragma unroll
+                for (int m = 0; m < SPL; ++m) {
+                    if (!(left >> m & 1u)) continue;
+                    const float3 l = xform_rows(r0, r1, r2, cx[m], cy[m], cz[m]);
+                    const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x);
+                    const float dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y);
+                    const float dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
+                    const float d2 = sq3(dx, dy, dz);
+                    if (d2 < cr[m] * cr[m]) c_box += cr[m] - sqrtf(d2);
+                }
+            }
+        }
+        // --- cylinders (finite, local z axis) ---
+        const float4 *cyl = bx + 5 * E.nb;
+#pragma unroll 1
+        for (int i = 0; i < nrc; ++i) {
+            if (!reached(nrs + nrb + i)) continue;
+            const int end = min(E.nc, (i + 1) * kWarp);
+#pragma unroll 1
+            for (int o = i * kWarp; o < end; ++o) {
+                const float4 r0 = cyl[4 * o], r1 = cyl[4 * o + 1], r2 = cyl[4 * o + 2], pr = cyl[4 * o + 3];
+#pragma unroll
+                for (int m = 0; m < SPL; ++m) {
+                    if (!(left >> m & 1u)) continue;
+                    const float3 l = xform_rows(r0, r1, r2, cx[m], cy[m], cz[m]);
+                    const float dx = sqrtf(__fmaf_rn(l.y, l.y, __fmul_rn(l.x, l.x))) - pr.x;
+                    const float dz = fabsf(l.z) - pr.y;
+                    const float ox = dx > 0.f ? dx : 0.f, oz = dz > 0.f ? dz : 0.f;
+                    const float outside = sqrtf(__fmaf_rn(oz, oz, __fmul_rn(ox, ox)));
+                    const float inside = fminf(fmaxf(dx, dz), 0.f);
+                    const float pen = cr[m] - (outside + inside);
+                    c_cyl += pen > 0.f ? pen : 0.f;
+                }
+            }
+        }
+    }
+
+    // --- self collision: group pairs whose bounding spheres overlap ---
+#pragma unroll 1
+    for (int k0 = 0; k0 < R.NPL; k0 += kWarp) {
+        const int k = k0 + lane;
+        bool on = false;
+        int p0 = 0, p1 = 0;
+        if (k < R.NPL) {
+            const int4 lp = t.lpair[k];
+            const float4 a = w.gb[pair_group(lp.x)], b = w.gb[pair_group(lp.y)];
+            const float rr = a.w + b.w;
+            on = sq3(a.x - b.x, a.y - b.y, a.z - b.z) < rr * rr;
+            p0 = lp.z;
+            p1 = lp.w;
+        }
+        unsigned bal = __ballot_sync(kFull, on);
+        while (bal) {
+            const int j = __ffs(bal) - 1;
+            bal &= bal - 1u;
+            const int q0 = __shfl_sync(kFull, p0, j), q1 = __shfl_sync(kFull, p1, j);
+            for (int p = q0 + lane; p < q1; p += kWarp) {
+                const unsigned ij = __ldg(R.pairs + p);
+                const float thr = __ldg(R.thr + p);
+                const float4 a = w.cen[ij & 0xffffu], b = w.cen[ij >> 16];
+                const float d2 = sq3(a.x - b.x, a.y - b.y, a.z - b.z);
+                if (d2 < thr) c_self += sqrtf(thr) - sqrtf(d2);
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        c_self += __shfl_xor_sync(kFull, c_self, off);
+        c_sph += __shfl_xor_sync(kFull, c_sph, off);
+        c_box += __shfl_xor_sync(kFull, c_box, off);
+        c_cyl += __shfl_xor_sync(kFull, c_cyl, off);
+    }
+    costs[0] = c_self; costs[1] = c_sph; costs[2] = c_box; costs[3] = c_cyl;
 }
 
 // Link poses [L*16] (row-major 4x4, last row 0 0 0 1) and sphere centres [S*3] of the
@@ -845,12 +946,11 @@ __device__ inline void store_fk(const SmemTables &t, const DevRobot &R, const Wa
     }
 }
 
-// One state of a collision check, one warp: FK of state s of q, its poses / centres when
-// asked for, the collision test, and the outputs (verdict; in cost mode the four
-// constraint costs [4][n] and their total).  k_check_costs and the batched check run
-// this routine, so their outputs are bit-identical.
-template <bool COST, int SPL>
-__device__ inline void check_state(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
+// State s of a cost check, one warp: FK of state s of q, its poses / centres when asked for,
+// the four constraint costs [4][n], their total and the verdict (a total that is not 0).
+// k_check_costs and the batched check run this routine, so their outputs are bit-identical.
+template <int SPL>
+__device__ inline void check_costs(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
                                    const float *__restrict__ q, long long s, long long n,
                                    unsigned char *__restrict__ verdict, float *__restrict__ costs,
                                    float *__restrict__ total, float *__restrict__ poses, float *__restrict__ centers,
@@ -859,18 +959,13 @@ __device__ inline void check_state(const SmemTables &t, const DevRobot &R, const
     __syncwarp();
     warp_fk(t, R.L, w, lane);
     if (poses || centers) store_fk(t, R, w, s, poses, centers, lane);
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool hit = (!COST && R.cull) ? warp_collide_culled<SPL>(t, R, E, w, lane)
-                                       : warp_collide<SPL, COST>(t, R, E, w, lane, c);
+    float c[4];
+    warp_costs<SPL>(t, R, E, w, lane, c);
     if (lane == 0) {
-        if (COST) {
-            const float tot = ((c[0] + c[1]) + c[2]) + c[3];
-            if (costs) { costs[s] = c[0]; costs[n + s] = c[1]; costs[2 * n + s] = c[2]; costs[3 * n + s] = c[3]; }
-            if (total) total[s] = tot;
-            if (verdict) verdict[s] = tot != 0.f;
-        } else if (verdict) {
-            verdict[s] = hit;
-        }
+        const float tot = ((c[0] + c[1]) + c[2]) + c[3];
+        if (costs) { costs[s] = c[0]; costs[n + s] = c[1]; costs[2 * n + s] = c[2]; costs[3 * n + s] = c[3]; }
+        if (total) total[s] = tot;
+        if (verdict) verdict[s] = tot != 0.f;
     }
     __syncwarp();
 }

@@ -214,7 +214,7 @@ __device__ bool block_edge_free(const SmemTables &t, const DevRobot &R, const De
             __syncwarp();
             warp_fk(t, R.L, w, lane);
             hit = CULL ? warp_collide_culled<SPL>(t, R, E, w, lane)
-                       : warp_collide<SPL, false>(t, R, E, w, lane, nullptr);
+                       : warp_collide<SPL>(t, R, E, w, lane);
         }
         if (hit && lane == 0) *s_flag = 1;
         __syncthreads();

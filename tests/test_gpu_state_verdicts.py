@@ -68,3 +68,36 @@ def test_a_scene_too_large_for_the_robot_is_refused():
     with pytest.raises(_lib.GbmpError) as e:
         _check(R, E, q)
     assert e.value.status == 5
+
+
+@pytest.mark.parametrize("n", [1, 33, 700, 60000])
+def test_costs(n):
+    """Costs against the oracle (a sample), and the same to the bit whatever states go
+    with a state: alone, in a batch request, or among many."""
+    robot = W.serial_arm(77, dof=8, n_spheres=90, prismatic_torso=True)
+    env = W.random_env(78, 150, 40, 12, oriented=True)
+    R, E, m = api.Robot(robot), api.Env(env), O.OracleModel(robot, env)
+    q = robot.sample_full(np.random.default_rng(n), n)
+    d = torch.from_numpy(q).cuda()
+    costs, total = torch.full((4, n), -1.0, device="cuda"), torch.full((n,), -1.0, device="cuda")
+    v = torch.full((n,), 9, dtype=torch.uint8, device="cuda")
+    api.check_states(R, E, d, v, costs, total, _lib.CHECK_COST)
+    pick = np.arange(n) if n <= 700 else np.random.default_rng(0).choice(n, 700, replace=False)
+    oc, ot = m.check_states(q[pick])
+    c, tt, vv = costs.cpu().numpy(), total.cpu().numpy(), v.cpu().numpy()
+    np.testing.assert_allclose(c[:, pick], oc, rtol=1e-4, atol=2e-5)
+    np.testing.assert_allclose(tt[pick], ot, rtol=1e-4, atol=2e-5)
+    np.testing.assert_array_equal(vv, tt != 0)
+    if n >= 700:
+        assert 0 < vv.sum() < n and all((c[k] > 0).any() for k in range(4))
+    at = min(n - 1, 5)
+    one, t1 = torch.zeros((4, 1), device="cuda"), torch.zeros(1, device="cuda")
+    api.check_states(R, E, d[at: at + 1].contiguous(), None, one, t1, _lib.CHECK_COST)
+    torch.cuda.synchronize()
+    assert torch.equal(one[:, 0], costs[:, at]) and torch.equal(t1[0], total[at])
+    cb = api.CheckBatch(max_requests=3)
+    few = d[: min(n, 301)].contiguous()
+    bc, bt = torch.zeros((4, len(few)), device="cuda"), torch.zeros(len(few), device="cuda")
+    cb.run([dict(robot=R, env=E, q=d[:1].contiguous()), dict(robot=R, env=E, q=few, costs=bc, total=bt)], mode=_lib.CHECK_COST)
+    torch.cuda.synchronize()
+    assert torch.equal(bc, costs[:, : len(few)]) and torch.equal(bt, total[: len(few)])
