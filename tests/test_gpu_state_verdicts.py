@@ -101,3 +101,18 @@ def test_costs(n):
     cb.run([dict(robot=R, env=E, q=d[:1].contiguous()), dict(robot=R, env=E, q=few, costs=bc, total=bt)], mode=_lib.CHECK_COST)
     torch.cuda.synchronize()
     assert torch.equal(bc, costs[:, : len(few)]) and torch.equal(bt, total[: len(few)])
+
+
+@pytest.mark.parametrize("cylinders", [0, 3])
+def test_states_that_are_no_numbers(cylinders):
+    """A state with a joint that is not a number: every distance comparison is false but a
+    cylinder's, whose clamps drop the NaN, so it collides just where there are cylinders."""
+    robot = W.serial_arm(79, dof=7, n_spheres=40)
+    R, E = api.Robot(robot), api.Env(W.random_env(80, 40, 8, cylinders, oriented=True))
+    q = torch.from_numpy(robot.sample_full(np.random.default_rng(2), 65)).cuda()
+    q[::2, 1] = float("nan")
+    v, total = torch.full((65,), 9, dtype=torch.uint8, device="cuda"), torch.zeros(65, device="cuda")
+    api.check_states(R, E, q, v, None, total, _lib.CHECK_COST)
+    torch.cuda.synchronize()
+    assert (v[::2] == (1 if cylinders else 0)).all()
+    np.testing.assert_array_equal(_check(R, E, q)[::2], v.cpu().numpy()[::2])
