@@ -195,7 +195,7 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
 }
 
 // ---------------------------------------------------------------------------------
-// FK alone (gbmp_fk): chunks of kFkChunk consecutive states per warp, the chunk FK above,
+// FK alone (gbmp_fk): chunks of up to kFkChunk consecutive states per warp, the chunk FK above,
 // then the chunk's link poses and sphere centres written out.  The poses of consecutive
 // states are consecutive in memory, so a chunk's poses are one block that the warp writes
 // as 16-byte words, 512 contiguous bytes per store (float4 rows from shared memory, the
@@ -203,27 +203,36 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
 // likewise one block, written lane by lane in order.
 // ---------------------------------------------------------------------------------
 constexpr int kFkChunk = 10;
+constexpr int kFkWarpBytes = 7680;
 
-__host__ __device__ inline size_t smem_fk_chunk_warp(const DevRobot &R) {
-    return align16(sizeof(float) * 12 * R.L * kFkChunk);
+// States of a chunk: ten up to 16 links, then as many as keep a warp's poses within
+// kFkWarpBytes (at least one).  More states a warp shorten the walk along the links per
+// state, fewer leave room for more warps: 199,277 states of a robot of 30 links (60 spheres)
+// take 210 us with 3, 194 with 4, 172 with 5, 179 with 7, 212 with 10; 314 us with a kernel
+// of one state a warp, which robots of more than 16 links had.
+inline int fk_chunk_states(const DevRobot &R) {
+    return std::max(1, std::min(kFkChunk, kFkWarpBytes / (int)(sizeof(float) * 12 * std::max(R.L, 1))));
+}
+__host__ __device__ inline size_t smem_fk_chunk_warp(const DevRobot &R, int kc) {
+    return align16(sizeof(float) * 12 * R.L * kc);
 }
 
 __global__ void __launch_bounds__(kChunkWarps *kWarp)
-    k_fk_chunk(DevRobot R, const float *__restrict__ q, long long n, float *__restrict__ poses,
+    k_fk_chunk(DevRobot R, const float *__restrict__ q, long long n, int kc, float *__restrict__ poses,
                float *__restrict__ centers, int vec) {
     extern __shared__ __align__(16) unsigned char smem[];
     const DevEnv E{};
     SmemTables t = carve_tables(smem, R, 0);
     if (!stage_tables(R, E, t, 0)) return;
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x & 31;
-    unsigned char *wbase = smem + smem_tables_bytes(R, 0) + smem_fk_chunk_warp(R) * warp;
+    unsigned char *wbase = smem + smem_tables_bytes(R, 0) + smem_fk_chunk_warp(R, kc) * warp;
     float *lpK = reinterpret_cast<float *>(wbase);
     const int L = R.L, S = R.S;
-    const long long nchunks = (n + kFkChunk - 1) / kFkChunk;
+    const long long nchunks = (n + kc - 1) / kc;
     const long long nw = (long long)gridDim.x * kChunkWarps;
     for (long long c = blockIdx.x * (long long)kChunkWarps + warp; c < nchunks; c += nw) {
-        const long long s0 = c * kFkChunk;
-        const int ks = (int)min((long long)kFkChunk, n - s0);
+        const long long s0 = c * kc;
+        const int ks = (int)min((long long)kc, n - s0);
         const float *qc = q + s0 * L;
         warp_fk_chunk_q<kFkChunk, 4>(t, L, ks, [&](int k, int i) { return qc[k * L + i]; }, lpK, lane);
         store_fk_states(t, L, S, lpK, s0, ks, poses, centers, vec, lane);
@@ -233,7 +242,8 @@ __global__ void __launch_bounds__(kChunkWarps *kWarp)
 
 gbmp_status fk_chunk_launch(const DevRobot &R, int num_sms, const float *q, long long n, float *poses,
                             float *centers, cudaStream_t s) {
-    const size_t smem = smem_tables_bytes(R, 0) + smem_fk_chunk_warp(R) * kChunkWarps;
+    const int kc = fk_chunk_states(R);
+    const size_t smem = smem_tables_bytes(R, 0) + smem_fk_chunk_warp(R, kc) * kChunkWarps;
     gbmp_status st = ensure_smem_optin((const void *)k_fk_chunk);
     if (st) return st;
     int per_sm = 0;
@@ -243,10 +253,10 @@ gbmp_status fk_chunk_launch(const DevRobot &R, int num_sms, const float *q, long
         return GBMP_ERR_CAPACITY;
     }
     long long grid = (long long)per_sm * num_sms;
-    const long long need = ((n + kFkChunk - 1) / kFkChunk + kChunkWarps - 1) / kChunkWarps;
+    const long long need = ((n + kc - 1) / kc + kChunkWarps - 1) / kChunkWarps;
     if (need < grid) grid = need;
     const int vec = (reinterpret_cast<uintptr_t>(poses) & 15u) == 0;
-    k_fk_chunk<<<(int)grid, kChunkWarps * kWarp, smem, s>>>(R, q, n, poses, centers, vec);
+    k_fk_chunk<<<(int)grid, kChunkWarps * kWarp, smem, s>>>(R, q, n, kc, poses, centers, vec);
     GBMP_CUDA(cudaGetLastError());
     return GBMP_OK;
 }

@@ -66,27 +66,6 @@ static gbmp_status persistent_grid(K kernel, size_t smem, int num_sms, int *grid
 // Kernels.
 // ---------------------------------------------------------------------------------
 
-// FK (+ sphere centres) of n states; one warp per state.
-__global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
-    k_fk(DevRobot R, const float *__restrict__ q, long long n, float *__restrict__ poses,
-         float *__restrict__ centers) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    DevEnv E{};
-    SmemTables t = carve_tables(smem, R, 0);
-    if (!stage_tables(R, E, t, 0)) return;
-    WarpScratch w = carve_warp(smem + smem_tables_bytes(R, 0), R, threadIdx.x / kWarp);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const long long nw = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long s = blockIdx.x * (long long)kWarpsPerBlock + threadIdx.x / kWarp; s < n; s += nw) {
-        for (int j = lane; j < R.L; j += kWarp) w.q[j] = q[s * R.L + j];
-        __syncwarp();
-        warp_fk(t, R.L, w, lane);
-        store_fk(t, R, w, s, poses, centers, lane);
-        __syncwarp();
-    }
-}
-
 // Costs of n states; one warp per state (warp_costs).  With poses / centers non-null the FK of
 // each state is also written out (the reference's update() and checkStates() from one FK).
 template <int SPL>
@@ -827,20 +806,8 @@ gbmp_status gbmp_fk(gbmp_robot r, const float *d_q, int64_t n, float *d_poses, f
     if (n == 0) return GBMP_OK;
     GBMP_CHECK_ARG(d_q, "q is NULL");
     if (r->use_cg) return codegen_fk(r, d_q, n, d_poses, d_centers, (cudaStream_t)stream);
-    if (r->dev.L <= 16) {
-        ProfScope ps(GBMP_PROF_FK, (cudaStream_t)stream);
-        return fk_chunk_launch(r->dev, r->num_sms, d_q, n, d_poses, d_centers, (cudaStream_t)stream);
-    }
-    const size_t smem = smem_tables_bytes(r->dev, 0) + smem_warp_bytes(r->dev) * kWarpsPerBlock;
-    int grid = 0;
-    gbmp_status st = persistent_grid(k_fk, smem, r->num_sms, &grid);
-    if (st) return st;
-    const long long need = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    if (need < grid) grid = (int)need;
     ProfScope ps(GBMP_PROF_FK, (cudaStream_t)stream);
-    k_fk<<<grid, kWarpsPerBlock * kWarp, smem, (cudaStream_t)stream>>>(r->dev, d_q, n, d_poses, d_centers);
-    GBMP_CUDA(cudaGetLastError());
-    return GBMP_OK;
+    return fk_chunk_launch(r->dev, r->num_sms, d_q, n, d_poses, d_centers, (cudaStream_t)stream);
 }
 
 gbmp_status gbmp_check_states_fk(gbmp_robot r, gbmp_env env, const float *d_q, int64_t n, int32_t mode,
