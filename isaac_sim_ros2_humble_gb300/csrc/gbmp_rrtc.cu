@@ -333,10 +333,15 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     if (s->dynamic_domain) p->dirty_radii[0] = p->dirty_radii[1] = p->cap;
 
     const DevEnv E = env->dev();
-    DevRobot DR = r->dev;
-    DR.work = nullptr;
     const int nwords = env_words(E.ns, E.nb, E.nc);
-    const size_t smem = rrtc_block_smem(DR, nwords, false);
+    // by chunks of states where the tables allow it (at most 32 groups) and the scratch fits
+    // next to the scene: faster at every lane count (the shelf at range 0.5: 1 lane 908 ->
+    // 530 us, 32 lanes 294 -> 156, 1,024 lanes 345 -> 163; at range 0.1: 2.45 -> 2.39 ms,
+    // 0.55 -> 0.52, 0.87 -> 0.65)
+    const bool chunk = r->dev_chunk.cull && rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk) <= kSmemLimit;
+    DevRobot DR = chunk ? r->dev_chunk : r->dev;
+    DR.work = nullptr;
+    const size_t smem = rrtc_block_smem(DR, nwords, chunk ? kRrtcSoloChunk : 0);
     RrtcParams prm;
     prm.lanes = s->lanes;
     prm.max_iters = s->max_iters;
@@ -359,8 +364,9 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     {
         ProfScope ps(GBMP_PROF_OTHER, st);
         const bool cull = DR.cull != 0;
-        const cudaError_t ce = DR.spl <= 4 ? rrtc_launch_lo(DR.spl, cull, s->lanes, smem, st, DR, E, D, prm)
-                                           : rrtc_launch_hi(DR.spl, cull, s->lanes, smem, st, DR, E, D, prm);
+        const cudaError_t ce = chunk         ? rrtc_launch_chunk(s->lanes, smem, st, DR, E, D, prm)
+                               : DR.spl <= 4 ? rrtc_launch_lo(DR.spl, cull, s->lanes, smem, st, DR, E, D, prm)
+                                             : rrtc_launch_hi(DR.spl, cull, s->lanes, smem, st, DR, E, D, prm);
         if (ce != cudaSuccess) {
             set_error("planning kernel launch (%zu bytes of shared memory): %s", smem, cudaGetErrorString(ce));
             stt = ce == cudaErrorInvalidValue ? GBMP_ERR_CAPACITY : GBMP_ERR_CUDA;
@@ -698,7 +704,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
         const DevEnv E = pr.env->dev();
         spl = std::max(spl, R.spl);
         cull = cull && R.cull;
-        smem = std::max(smem, rrtc_block_smem(R, env_words(E.ns, E.nb, E.nc), true));
+        smem = std::max(smem, rrtc_block_smem(R, env_words(E.ns, E.nb, E.nc), kRrtcChunk));
         BatchProblem &bp = b->h_table[i];
         bp.R = R;
         bp.R.work = nullptr;

@@ -11,18 +11,20 @@ namespace gbmp {
 
 constexpr int kRrtcWarps = 4;
 constexpr int kRrtcThreads = kRrtcWarps * kWarp;
-// States per chunk of the planner's edge checks: an extension of at most `range` has a
-// dozen states or so, split over the lane's four warps, so chunks stay small (and so
-// does the per-warp chunk scratch in shared memory).
+// States per chunk of the planner's edge checks, batched and for one problem: an extension
+// of at most `range` has a dozen states or so, split over the lane's four warps, so chunks
+// stay small (and so does the per-warp chunk scratch in shared memory).  One lane on the
+// shelf at range 0.5, 25 states an edge: 546 us a problem with 4, 530 with 8, 528 with 10.
 constexpr int kRrtcChunk = 4;
+constexpr int kRrtcSoloChunk = 8;
 
 // Shared memory of a planning block: staged tables, four warp scratches, the lane's
-// joint vectors and flags, and, when the edge checks run by chunks (batched planning,
-// robots of at most 32 sphere groups), four chunk scratches.
+// joint vectors and flags, and, when the edge checks run by chunks of `chunk` states
+// (robots of at most 32 sphere groups), four chunk scratches.
 __host__ __device__ inline size_t rrtc_misc_bytes() { return align16(6 * kMaxLinks * 4 + 256); }
-__host__ __device__ inline size_t rrtc_block_smem(const DevRobot &R, int nwords, bool chunks) {
+__host__ __device__ inline size_t rrtc_block_smem(const DevRobot &R, int nwords, int chunk) {
     return smem_tables_bytes(R, nwords) + smem_warp_bytes(R) * kRrtcWarps + rrtc_misc_bytes() +
-           (chunks && R.cull ? smem_chunk_bytes(R, kRrtcChunk) * kRrtcWarps : 0);
+           (chunk && R.cull ? smem_chunk_bytes(R, chunk) * kRrtcWarps : 0);
 }
 
 enum : int { kStRunning = 0, kStSolved = 1, kStNodeCap = 2, kStIterCap = 3, kStDeadline = 4 };
@@ -111,6 +113,8 @@ cudaError_t rrtc_launch_lo(int spl, bool cull, int grid, size_t smem, cudaStream
                            const DevEnv &E, const RrtcDev &P, const RrtcParams &prm);
 cudaError_t rrtc_launch_hi(int spl, bool cull, int grid, size_t smem, cudaStream_t st, const DevRobot &R,
                            const DevEnv &E, const RrtcDev &P, const RrtcParams &prm);
+cudaError_t rrtc_launch_chunk(int grid, size_t smem, cudaStream_t st, const DevRobot &R, const DevEnv &E,
+                            const RrtcDev &P, const RrtcParams &prm);
 cudaError_t rrtc_batch_launch_lo(int spl, bool cull, int grid, size_t smem, cudaStream_t st,
                                  const BatchProblem *probs, int n, int lanes_per_problem, const RrtcParams &prm,
                                  int *rr);

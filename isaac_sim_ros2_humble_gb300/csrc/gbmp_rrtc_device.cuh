@@ -148,15 +148,12 @@ __device__ inline int block_nearest(const float *__restrict__ nodes, int size, i
 // states of one direction and on a state of the other.  old_first: a is the node already
 // in the tree (start tree edges), state 0 (= a) is skipped unless n == 1; otherwise
 // (goal tree edges, the new node first) b is the node already in the tree and the last
-// state (= b) is skipped, and with n == 1 the one state checked is a.  CHUNK (batched
-// planning, robots of at most 32 sphere groups): the states are split into chunks of
+// state (= b) is skipped, and with n == 1 the one state checked is a.  CHUNK > 0
+// (robots of at most 32 sphere groups): the states are split into chunks of up to CHUNK
 // consecutive states, one chunk per warp at a time, each with one broad phase for its
-// states (warp_edge_chunk, whose narrow tests are the per-state ones): measured 487
-// against 531 ms on the uneven batch, whose time is the trees of the problems without a
-// path growing to their node cap.  Otherwise one warp per state, which keeps the
-// single-problem kernel at 5 blocks per SM (its p50 time to solution is 4 % longer with
-// chunks).  Returns true if every state is collision-free.
-template <int SPL, bool CULL, bool CHUNK>
+// states (warp_edge_chunk, whose narrow tests are the per-state ones).  Otherwise one warp
+// per state.  Returns true if every state is collision-free.
+template <int SPL, bool CULL, int CHUNK>
 __device__ bool block_edge_free(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
                                 const ChunkScratch &cs, const float *a, const float *b,
                                 float res, int rule, bool old_first, int *s_flag, float *s_dir, int *s_n) {
@@ -186,41 +183,41 @@ __device__ bool block_edge_free(const SmemTables &t, const DevRobot &R, const De
     __syncthreads();
     const int first = old_first ? (n == 1 ? 0 : 1) : 0;
     const int last = old_first ? n : (n == 1 ? 1 : n - 1);   // exclusive
-    if (CULL && CHUNK) {
+    if constexpr (CULL && CHUNK > 0) {
         // chunks of `per` states; warp v takes chunk v of every round of four.  The chunk
         // routine replaces state n - 1 by b; the new-node-first single state is a, so it
         // runs as state 0 of two
         const int nstates = (!old_first && n == 1) ? 2 : n;
-        const int per = min(kRrtcChunk, (last - first + kRrtcWarps - 1) / kRrtcWarps);
+        const int per = min(CHUNK, (last - first + kRrtcWarps - 1) / kRrtcWarps);
         for (int c0 = first; c0 < last; c0 += per * kRrtcWarps) {
             const int s0 = c0 + warp * per, s1 = min(s0 + per, last);
             int h = -1;
             if (s0 < s1)
-                h = warp_edge_chunk<kRrtcChunk, false>(t, R, E, cs, lane, a, b, s_dir, s0, s1, nstates, true);
+                h = warp_edge_chunk<CHUNK, false>(t, R, E, cs, lane, a, b, s_dir, s0, s1, nstates, true);
             if (h >= 0 && lane == 0) *s_flag = 1;
             __syncthreads();
             const bool any = *s_flag != 0;
             __syncthreads();
             if (any) return false;
         }
-        return true;
-    }
-    for (int k0 = first; k0 < last; k0 += kRrtcWarps) {
-        const int k = k0 + warp;
-        bool hit = false;
-        if (k < last) {
-            for (int j = lane; j < R.L; j += kWarp)
-                w.q[j] = (old_first && k == n - 1) ? b[j] : __fmaf_rn(s_dir[j], (float)k, a[j]);
-            __syncwarp();
-            warp_fk(t, R.L, w, lane);
-            hit = CULL ? warp_collide_culled<SPL>(t, R, E, w, lane)
-                       : warp_collide<SPL>(t, R, E, w, lane);
+    } else {
+        for (int k0 = first; k0 < last; k0 += kRrtcWarps) {
+            const int k = k0 + warp;
+            bool hit = false;
+            if (k < last) {
+                for (int j = lane; j < R.L; j += kWarp)
+                    w.q[j] = (old_first && k == n - 1) ? b[j] : __fmaf_rn(s_dir[j], (float)k, a[j]);
+                __syncwarp();
+                warp_fk(t, R.L, w, lane);
+                hit = CULL ? warp_collide_culled<SPL>(t, R, E, w, lane)
+                           : warp_collide<SPL>(t, R, E, w, lane);
+            }
+            if (hit && lane == 0) *s_flag = 1;
+            __syncthreads();
+            const bool any = *s_flag != 0;
+            __syncthreads();
+            if (any) return false;
         }
-        if (hit && lane == 0) *s_flag = 1;
-        __syncthreads();
-        const bool any = *s_flag != 0;
-        __syncthreads();
-        if (any) return false;
     }
     return true;
 }
@@ -275,7 +272,7 @@ __device__ inline void publish_end(const RrtcDev &P, int value) {
 
 // One extension lane of one problem (the body of both the single-problem and the
 // batched planning kernels).  All threads of the block call it.
-template <int SPL, bool CULL, bool CHUNK>
+template <int SPL, bool CULL, int CHUNK>
 __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, const RrtcParams &prm,
                           const int lane_id) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -295,7 +292,7 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
     int *s_misc = s_i + kRrtcWarps;                      // [8]
     unsigned char *act = reinterpret_cast<unsigned char *>(s_misc + 8);
     ChunkScratch cs{};
-    if (CULL && CHUNK) carve_chunk(p + rrtc_misc_bytes(), R, kRrtcChunk, threadIdx.x / kWarp, cs);
+    if (CULL && CHUNK > 0) carve_chunk(p + rrtc_misc_bytes(), R, CHUNK, threadIdx.x / kWarp, cs);
     for (int j = threadIdx.x; j < R.L; j += blockDim.x) act[j] = R.active[j];
     __syncthreads();
 
@@ -435,7 +432,7 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
 
 template <int SPL, bool CULL>
 __global__ void __launch_bounds__(kRrtcThreads, 5) k_rrtc(DevRobot R, DevEnv E, RrtcDev P, RrtcParams prm) {
-    rrtc_lane<SPL, CULL, false>(R, E, P, prm, blockIdx.x);
+    rrtc_lane<SPL, CULL, 0>(R, E, P, prm, blockIdx.x);
 }
 
 // Batched planning: block b serves problem b % n as lane b / n, so every problem gets
@@ -467,7 +464,7 @@ __global__ void __launch_bounds__(kRrtcThreads, 4) k_rrtc_batch(const BatchProbl
         RrtcParams q = prm;
         q.lanes = lanes_per_problem;
         q.seed = sSeed;
-        rrtc_lane<SPL, CULL, CULL>(sR, sE, sP, q, sLane);
+        rrtc_lane<SPL, CULL, CULL ? kRrtcChunk : 0>(sR, sE, sP, q, sLane);
         __syncthreads();
         if (threadIdx.x == 0) {
             // the last lane to leave an ended, unsolved problem publishes its end
