@@ -101,7 +101,8 @@ struct gbmp_check_batch_s {
     int device = 0, num_sms = 0, max_requests = 0, max_ranges = 0;
     unsigned char *h_buf = nullptr;   // pinned: tasks, then ranges
     unsigned char *d_buf = nullptr;
-    size_t ranges_off = 0, bytes = 0;
+    size_t bytes = 0;
+    std::vector<int> order;           // the requests of a call that have states, as they are listed
     cudaEvent_t uploaded = nullptr;   // the last upload from h_buf has been read
     bool pending = false;
 };
@@ -124,8 +125,7 @@ gbmp_status gbmp_check_batch_create(int32_t max_requests, gbmp_check_batch *out)
             break;
         }
         b->max_ranges = max_requests + kBatchBlocksPerSm * b->num_sms;
-        b->ranges_off = align16(sizeof(CheckTask) * (size_t)max_requests);
-        b->bytes = b->ranges_off + sizeof(CheckRange) * (size_t)b->max_ranges;
+        b->bytes = align16(sizeof(CheckTask) * (size_t)max_requests) + sizeof(CheckRange) * (size_t)b->max_ranges;
         if (cudaMallocHost(&b->h_buf, b->bytes) != cudaSuccess || cudaMalloc(&b->d_buf, b->bytes) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming) != cudaSuccess) {
             set_error("check batch: allocation of %zu bytes failed", b->bytes);
@@ -175,7 +175,18 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         b->pending = false;
     }
     auto *tasks = reinterpret_cast<CheckTask *>(b->h_buf);
-    auto *ranges = reinterpret_cast<CheckRange *>(b->h_buf + b->ranges_off);
+    // requests of one robot and scene next to each other, so that the blocks the GPU
+    // schedules together share their tables (in L2) and their path through the routine
+    // (measured 5.74 against 6.05 ms on the 256-request benchmark mix); sorted by their
+    // numbers, for a task is half a kilobyte
+    b->order.clear();
+    for (int i = 0; i < n_reqs; ++i)
+        if (reqs[i].n) b->order.push_back(i);
+    std::stable_sort(b->order.begin(), b->order.end(), [reqs](int x, int y) {
+        const gbmp_check_request &p = reqs[x], &q = reqs[y];
+        if (p.robot != q.robot) return p.robot->dev.stage < q.robot->dev.stage;
+        return p.env->view.words < q.env->view.words;
+    });
     const bool cost = mode == GBMP_CHECK_COST;
     int nt = 0, spl = 1;
     size_t smem = 0;   // of the costs' kernel, which also says which requests fit
@@ -183,9 +194,8 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
     DevRobot widest{};
     long long total = 0;
     unsigned long long *work = work_counter();
-    for (int i = 0; i < n_reqs; ++i) {
+    for (int i : b->order) {
         const gbmp_check_request &q = reqs[i];
-        if (q.n == 0) continue;
         CheckTask &T = tasks[nt++];
         T.R = cost ? q.robot->dev : q.robot->dev_chunk;
         T.R.work = work;
@@ -206,13 +216,6 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         total += q.n;
     }
     if (nt == 0) return GBMP_OK;
-    // requests of one robot and scene next to each other, so that the blocks the GPU
-    // schedules together share their tables (in L2) and their path through the routine
-    // (measured 5.74 against 6.05 ms on the 256-request benchmark mix)
-    std::stable_sort(tasks, tasks + nt, [](const CheckTask &x, const CheckTask &y) {
-        if (x.R.stage != y.R.stage) return x.R.stage < y.R.stage;
-        return x.E.words < y.E.words;
-    });
     int optin = 0;
     GBMP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     if (smem + 1024 > (size_t)optin) {
@@ -250,6 +253,8 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
     long long spb = (total + target - 1) / target;
     spb = std::max<long long>(spb, cost ? 4 * unit : unit);   // costs: at least four states a warp
     spb = (spb + unit - 1) / unit * unit;
+    const size_t ranges_off = align16(sizeof(CheckTask) * (size_t)nt);   // the ranges follow the tasks: one copy
+    auto *ranges = reinterpret_cast<CheckRange *>(b->h_buf + ranges_off);
     int nr = 0;
     for (int ti = 0; ti < nt; ++ti)
         for (long long lo = 0; lo < tasks[ti].n; lo += spb) {
@@ -259,19 +264,11 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
             }
             ranges[nr++] = CheckRange{ti, 0, lo, std::min(lo + spb, tasks[ti].n)};
         }
-    // tasks and ranges in one copy (the ranges follow the tasks at ranges_off)
-    const size_t nbytes = b->ranges_off + sizeof(CheckRange) * (size_t)nr;
-    if (b->ranges_off > sizeof(CheckTask) * (size_t)nt) {
-        GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, sizeof(CheckTask) * (size_t)nt, cudaMemcpyHostToDevice, s));
-        GBMP_CUDA(cudaMemcpyAsync(b->d_buf + b->ranges_off, b->h_buf + b->ranges_off, sizeof(CheckRange) * (size_t)nr,
-                                  cudaMemcpyHostToDevice, s));
-    } else {
-        GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, nbytes, cudaMemcpyHostToDevice, s));
-    }
+    GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, ranges_off + sizeof(CheckRange) * (size_t)nr, cudaMemcpyHostToDevice, s));
     GBMP_CUDA(cudaEventRecord(b->uploaded, s));
     b->pending = true;
     const auto *d_tasks = reinterpret_cast<const CheckTask *>(b->d_buf);
-    const auto *d_ranges = reinterpret_cast<const CheckRange *>(b->d_buf + b->ranges_off);
+    const auto *d_ranges = reinterpret_cast<const CheckRange *>(b->d_buf + ranges_off);
     ProfScope ps(GBMP_PROF_CHECK_STATES, s);
     void *args[] = {&d_tasks, &d_ranges, &sh.ks};   // the costs' kernel takes the first two
     GBMP_CUDA(cudaLaunchKernel(fn, dim3(nr), dim3(sh.warps * kWarp), args, sh.smem, s));
