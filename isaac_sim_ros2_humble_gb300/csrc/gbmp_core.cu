@@ -109,11 +109,10 @@ __global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStates
 // edge.  Also counts the edges per length bucket (hist, longest bucket first) for the
 // longest-first processing order.  An edge of more than kMaxEdgeStates states gets
 // kMaxEdgeStates + 1 and is not validated.
-__global__ void k_edge_setup(const float *__restrict__ from, const float *__restrict__ to, long long E, int L,
-                             float res, int rule, int *__restrict__ nsteps, float *__restrict__ dir,
-                             int *__restrict__ hist, float *__restrict__ length_out, int *__restrict__ nsteps_out) {
-    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (k >= E) return;
+__device__ __forceinline__ int edge_setup(const float *__restrict__ from, const float *__restrict__ to, long long k,
+                                          int L, float res, int rule, int *__restrict__ nsteps,
+                                          float *__restrict__ dir, float *__restrict__ length_out,
+                                          int *__restrict__ nsteps_out) {
     const float *f = from + k * L, *t = to + k * L;
     float d2 = 0.f, dinf = 0.f;
     for (int j = 0; j < L; ++j) {
@@ -131,9 +130,17 @@ __global__ void k_edge_setup(const float *__restrict__ from, const float *__rest
     const float fn = count ? (float)(n - 1) : (float)n;
     for (int j = 0; j < L; ++j) dir[k * L + j] = __fdiv_rn(__fadd_rn(t[j], -f[j]), fn);
     nsteps[k] = n;
-    atomicAdd(hist + edge_bucket(n), 1);
     if (length_out) length_out[k] = len;
     if (nsteps_out) nsteps_out[k] = n;
+    return n;
+}
+
+__global__ void k_edge_setup(const float *__restrict__ from, const float *__restrict__ to, long long E, int L,
+                             float res, int rule, int *__restrict__ nsteps, float *__restrict__ dir,
+                             int *__restrict__ hist, float *__restrict__ length_out, int *__restrict__ nsteps_out) {
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k >= E) return;
+    atomicAdd(hist + edge_bucket(edge_setup(from, to, k, L, res, rule, nsteps, dir, length_out, nsteps_out)), 1);
 }
 
 // Processing order of the edges, longest bucket first: order[slot] = edge, the slots of a
@@ -148,44 +155,81 @@ __global__ void k_edge_setup(const float *__restrict__ from, const float *__rest
 // 2.32 with 16, 2.45 with 8; 17,339 shorter edges 0.312, 0.318 and 0.373 ms; 4 or 16 items
 // a warp instead of 8 cost up to 10 % on batches of 17,000 to 33,000 edges).
 constexpr int kItemsPerWarp = 8, kGrabsPerWarp = 32, kMaxSpan = 8;
+// First place of every bucket in the order, from the buckets' counts; and, where `plan` is
+// given, the plan of parts.  One warp.
+__device__ __forceinline__ void edge_plan(const int *hist, long long E, int K, int warps, int *base,
+                                          EdgePlan *__restrict__ plan, int lane) {
+    static_assert(kEdgeBuckets == 2 * kWarp, "two buckets a lane");
+    const int b0 = 2 * lane;
+    const int h0 = hist[b0], h1 = hist[b0 + 1];
+    int acc = h0 + h1;   // edges up to this lane's buckets
+    for (int off = 1; off < kWarp; off <<= 1) {
+        const int v = __shfl_up_sync(kFull, acc, off);
+        if (lane >= off) acc += v;
+    }
+    base[b0] = acc - h1 - h0;
+    base[b0 + 1] = acc - h1;
+    if (!K || !plan) return;
+    // chunks of an edge of bucket b: about (16 (63 - b) + 8) / K
+    float chunks = (float)h0 * (1 + (16 * (kEdgeBuckets - 1 - b0) + 8) / K) +
+                   (float)h1 * (1 + (16 * (kEdgeBuckets - 2 - b0) + 8) / K);
+    for (int off = 16; off; off >>= 1) chunks += __shfl_xor_sync(kFull, chunks, off);
+    const int first = __ffs(__ballot_sync(kFull, h0 + h1 > 0)) - 1;   // E > 0: some bucket holds an edge
+    const int longest = 2 * first + (__shfl_sync(kFull, h0, first) ? 0 : 1);
+    if (lane == 0) {
+        const int most = 2 + 16 * (kEdgeBuckets - longest) / K;   // chunks of the longest edge (longer: bucket 0)
+        const int span = max(1, min(kMaxSpan, (int)(chunks / (4.f * kItemsPerWarp * warps))));
+        const int parts = max(1, min(kEdgeMaxParts, (most + span - 1) / span));
+        const int grab = (int)max(1LL, min(32LL, E * parts / ((long long)kGrabsPerWarp * warps)));
+        *plan = EdgePlan{parts, span, grab, parts > 1 && E < warps, E < 2 * warps};
+    }
+}
+
+// Edge k of n states: its place in the order, and its outputs without a collision.
+__device__ __forceinline__ void edge_place(long long k, int n, int place, int *__restrict__ order,
+                                           unsigned char *__restrict__ ok, int *__restrict__ first_hit) {
+    order[place] = (int)k;
+    if (ok) ok[k] = n <= kMaxEdgeStates;
+    if (first_hit) first_hit[k] = n <= kMaxEdgeStates ? -1 : -2;
+}
+
 __global__ void k_edge_order(const int *__restrict__ nsteps, long long E, const int *__restrict__ hist,
                              int *__restrict__ cursor, int *__restrict__ order, unsigned char *__restrict__ ok,
                              int *__restrict__ first_hit, int K, int warps, EdgePlan *__restrict__ plan) {
     __shared__ int base[kEdgeBuckets];
-    static_assert(kEdgeBuckets == 2 * kWarp, "two buckets a lane");
-    if (threadIdx.x < kWarp) {
-        const int lane = threadIdx.x, b0 = 2 * lane;
-        const int h0 = hist[b0], h1 = hist[b0 + 1];
-        int acc = h0 + h1;   // edges up to this lane's buckets
-        for (int off = 1; off < kWarp; off <<= 1) {
-            const int v = __shfl_up_sync(kFull, acc, off);
-            if (lane >= off) acc += v;
-        }
-        base[b0] = acc - h1 - h0;
-        base[b0 + 1] = acc - h1;
-        if (K && blockIdx.x == 0) {
-            // chunks of an edge of bucket b: about (16 (63 - b) + 8) / K
-            float chunks = (float)h0 * (1 + (16 * (kEdgeBuckets - 1 - b0) + 8) / K) +
-                           (float)h1 * (1 + (16 * (kEdgeBuckets - 2 - b0) + 8) / K);
-            for (int off = 16; off; off >>= 1) chunks += __shfl_xor_sync(kFull, chunks, off);
-            const int first = __ffs(__ballot_sync(kFull, h0 + h1 > 0)) - 1;   // E > 0: some bucket holds an edge
-            const int longest = 2 * first + (__shfl_sync(kFull, h0, first) ? 0 : 1);
-            if (lane == 0) {
-                const int most = 2 + 16 * (kEdgeBuckets - longest) / K;   // chunks of the longest edge (longer: bucket 0)
-                const int span = max(1, min(kMaxSpan, (int)(chunks / (4.f * kItemsPerWarp * warps))));
-                const int parts = max(1, min(kEdgeMaxParts, (most + span - 1) / span));
-                const int grab = (int)max(1LL, min(32LL, E * parts / ((long long)kGrabsPerWarp * warps)));
-                *plan = EdgePlan{parts, span, grab, parts > 1 && E < warps, E < 2 * warps};
-            }
-        }
-    }
+    if (threadIdx.x < kWarp) edge_plan(hist, E, K, warps, base, blockIdx.x == 0 ? plan : nullptr, threadIdx.x);
     __syncthreads();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < E; k += (long long)gridDim.x * blockDim.x) {
         const int n = nsteps[k], b = edge_bucket(n);
-        order[base[b] + atomicAdd(cursor + b, 1)] = (int)k;
-        if (ok) ok[k] = n <= kMaxEdgeStates;
-        if (first_hit) first_hit[k] = n <= kMaxEdgeStates ? -1 : -2;
+        edge_place(k, n, base[b] + atomicAdd(cursor + b, 1), order, ok, first_hit);
     }
+}
+
+// Set-up, order and plan of at most kFewEdges edges by one block, a thread an edge, the
+// buckets' counts in shared memory: one launch where k_edge_setup and k_edge_order with the
+// zeroing of their counters are three (64 edges: 37 us a call, 41 with
+// the three).
+constexpr int kFewEdges = 1024;
+__global__ void __launch_bounds__(kFewEdges)
+    k_edge_few(const float *__restrict__ from, const float *__restrict__ to, int E, int L, float res, int rule,
+               int *__restrict__ nsteps, float *__restrict__ dir, float *__restrict__ length_out,
+               int *__restrict__ nsteps_out, int *__restrict__ order, unsigned char *__restrict__ ok,
+               int *__restrict__ first_hit, int K, int warps, EdgePlan *__restrict__ plan,
+               unsigned long long *__restrict__ next) {
+    __shared__ int hist[kEdgeBuckets], base[kEdgeBuckets];
+    for (int b = threadIdx.x; b < kEdgeBuckets; b += blockDim.x) hist[b] = 0;
+    if (threadIdx.x == 0) *next = 0ull;
+    __syncthreads();
+    const int k = threadIdx.x;
+    int n = 0, at = 0;
+    if (k < E) {
+        n = edge_setup(from, to, k, L, res, rule, nsteps, dir, length_out, nsteps_out);
+        at = atomicAdd(hist + edge_bucket(n), 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < kWarp) edge_plan(hist, E, K, warps, base, plan, threadIdx.x);
+    __syncthreads();
+    if (k < E) edge_place(k, n, base[edge_bucket(n)] + at, order, ok, first_hit);
 }
 
 // Edge validation state by state (robots with more than 32 sphere groups, and the
@@ -937,18 +981,22 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
     EdgePlan *plan = reinterpret_cast<EdgePlan *>(next + 4);   // next: 8 bytes, 16-byte aligned
     float *dir = sc.dir;
     const int L = r->L;
-    GBMP_CUDA(cudaMemsetAsync(ctr, 0, kEdgeCtrInts * sizeof(int), s));
     const int tb = 256;
     const unsigned blocks = (unsigned)((E + tb - 1) / tb);
+    const bool own = !r->use_cg || rule == GBMP_STEP_COUNT;   // the generated set-up knows the checkMotions rules
+    const bool few = own && E <= kFewEdges;
     gbmp_status st = GBMP_OK;
-    if (r->use_cg && rule != GBMP_STEP_COUNT) {   // the generated set-up knows the checkMotions rules
-        st = codegen_edge_setup(r, d_from, d_to, E, res, rule, nsteps, dir, hist, d_length, d_num_steps, s);
-        if (st) return st;
-    } else {
-        ProfScope ps(GBMP_PROF_OTHER, s);
-        k_edge_setup<<<blocks, tb, 0, s>>>(d_from, d_to, E, L, res, rule, nsteps, dir, hist, d_length, d_num_steps);
+    if (!few) {
+        GBMP_CUDA(cudaMemsetAsync(ctr, 0, kEdgeCtrInts * sizeof(int), s));
+        if (own) {
+            ProfScope ps(GBMP_PROF_OTHER, s);
+            k_edge_setup<<<blocks, tb, 0, s>>>(d_from, d_to, E, L, res, rule, nsteps, dir, hist, d_length, d_num_steps);
+        } else {
+            st = codegen_edge_setup(r, d_from, d_to, E, res, rule, nsteps, dir, hist, d_length, d_num_steps, s);
+            if (st) return st;
+        }
+        GBMP_CUDA(cudaGetLastError());
     }
-    GBMP_CUDA(cudaGetLastError());
     const DevEnv Ev = env->dev();
     DevRobot D = r->dev;
     D.work = work_counter();
@@ -976,8 +1024,13 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
     if (st) return st;
     {
         ProfScope ps(GBMP_PROF_OTHER, s);
-        k_edge_order<<<(unsigned)std::min<long long>(blocks, 4LL * r->num_sms), tb, 0, s>>>(
-            nsteps, E, hist, cursor, order, d_ok, d_first_hit, K, edge_chunk_warps(grid), plan);
+        if (few)
+            k_edge_few<<<1, (unsigned)((E + kWarp - 1) / kWarp * kWarp), 0, s>>>(
+                d_from, d_to, (int)E, L, res, rule, nsteps, dir, d_length, d_num_steps, order, d_ok, d_first_hit, K,
+                edge_chunk_warps(grid), plan, reinterpret_cast<unsigned long long *>(next));
+        else
+            k_edge_order<<<(unsigned)std::min<long long>(blocks, 4LL * r->num_sms), tb, 0, s>>>(
+                nsteps, E, hist, cursor, order, d_ok, d_first_hit, K, edge_chunk_warps(grid), plan);
     }
     GBMP_CUDA(cudaGetLastError());
     if (!K) {   // one warp per edge at most

@@ -186,7 +186,7 @@ int edge_chunk_warps(int grid);
 // chunk for this robot (0: use the per-state kernels); `form` is the robot handle's
 // edge_form (0 automatic, 1 per state, 4 or 10 states per chunk).
 int edge_chunk_states(const DevRobot &R, int form);
-// FK alone of n states by chunks of consecutive states (robots of at most 16 links).
+// FK alone of n states by chunks of consecutive states.
 gbmp_status fk_chunk_launch(const DevRobot &R, int num_sms, const float *q, long long n, float *poses,
                             float *centers, cudaStream_t s);
 gbmp_status edge_chunk_prepare(const DevRobot &R, const DevEnv &E, int num_sms, int K, size_t *smem, int *grid);

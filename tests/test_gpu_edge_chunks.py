@@ -6,7 +6,7 @@ import dataclasses
 import numpy as np
 import pytest
 
-from isaac_sim_ros2_humble_gb300 import api, workloads as W
+from isaac_sim_ros2_humble_gb300 import _lib, api, workloads as W
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -120,3 +120,26 @@ def test_batches_whose_edges_are_settled_by_their_probes(n):
             np.testing.assert_array_equal(got[0], want[0])
             np.testing.assert_array_equal(got[1], want[1])
             np.testing.assert_array_equal(_run(R, E, a, b, 0.01, False)[0], want[0])
+
+
+@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025])
+def test_few_edges_as_among_many(n, form):
+    """Up to 1,024 edges are prepared by one block: every output as in a batch of 3,000."""
+    robot = W.serial_arm(95, dof=7, n_spheres=50)
+    R, E = api.Robot(robot), api.Env(W.random_env(96, 60, 8, 4, oriented=True))
+    R.set_edge_form(form)
+    g = np.random.default_rng(7)
+    a, b = (torch.from_numpy(robot.sample_full(g, 3000)).cuda() for _ in range(2))
+    b[::17] = a[::17]                      # edges of one state
+    b[5, 2] = float("inf")                 # an edge too long to validate
+
+    def check(k):
+        ok, length = torch.full((k,), 7, dtype=torch.uint8, device="cuda"), torch.zeros(k, device="cuda")
+        hit, steps = (torch.full((k,), 9, dtype=torch.int32, device="cuda") for _ in range(2))
+        api.check_edges(R, E, a[:k].contiguous(), b[:k].contiguous(), 0.05, _lib.STEP_LINF, ok, hit, length, steps)
+        torch.cuda.synchronize()
+        return ok, hit, length, steps
+
+    for few, many in zip(check(n), check(3000)):
+        assert torch.equal(few, many[:n])
