@@ -780,26 +780,30 @@ __device__ inline bool warp_collide_culled(const SmemTables &t, const DevRobot &
 // EnvConstraintCylinder.cu:130-180, summed over the pairs that can touch.  A sphere that the
 // scene's field clears takes part in no scene term, nor does a run of 32 obstacles that no
 // sphere left reaches; self pairs go by group pairs whose spheres overlap.  What is passed
-// over adds nothing: every term of it is 0.  Summing all pairs (336 obstacles x 110 spheres
-// and 3,192 self pairs a state) took 628 us for 20,011 states, 222 us now.
+// over adds nothing: every term of it is 0.  The spheres left are listed, up to 32 at a time,
+// and go one a lane against one obstacle after another, or, fewer than kTogether of them, one
+// after another against an obstacle a lane.  Summing all pairs (336 obstacles x 110 spheres
+// and 3,192 self pairs a state) took 628 us for 20,011 states; each lane's own four spheres
+// with this culling 225 us; listed 165 us (172 when a sphere always has a lane, 287 when it
+// never has; lists of 5 or 16 as the line between the two: 166).
+constexpr int kTogether = 10;
 template <int SPL>
 __device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
                                   int lane, float *costs) {
-    float cx[SPL], cy[SPL], cz[SPL], cr[SPL];
-    unsigned left = 0u;   // bit m: some lane's sphere m is left
+    unsigned near[SPL];   // lanes whose sphere lane + 32 m the field leaves
+    int nnear = 0;
 #pragma unroll
     for (int m = 0; m < SPL; ++m) {
         const int k = lane + kWarp * m;
-        cx[m] = kFar; cy[m] = kFar; cz[m] = kFar; cr[m] = 0.f;
-        bool near = false;
+        bool on = false;
         if (k < R.S) {
             const float4 s = t.sph[k];
             const float3 p = xform_point(w.lp + 12 * t.slink[k], s.x, s.y, s.z);
             w.cen[k] = make_float4(p.x, p.y, p.z, s.w);
-            near = !scene_far(E, p.x, p.y, p.z, s.w + kBroadMargin);
-            if (near) { cx[m] = p.x; cy[m] = p.y; cz[m] = p.z; cr[m] = s.w; }
+            on = !scene_far(E, p.x, p.y, p.z, s.w + kBroadMargin);
         }
-        left |= __any_sync(kFull, near) ? 1u << m : 0u;
+        near[m] = __ballot_sync(kFull, on);
+        nnear += __popc(near[m]);
     }
     for (int g = lane; g < R.G; g += kWarp) {
         const float4 s = t.grp[g];
@@ -809,81 +813,82 @@ __device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const 
     __syncwarp();
 
     float c_self = 0.f, c_sph = 0.f, c_box = 0.f, c_cyl = 0.f;
+    const int nrs = env_clusters(E.ns), nrb = env_clusters(E.nb), nrun = nrs + nrb + env_clusters(E.nc);
     const float4 *runs = t.env + env_cluster_base(E.ns, E.nb, E.nc);
-    // whether some sphere left reaches run i
-    auto reached = [&](int i) {
+    // whether the sphere (x, y, z, r) reaches run i (a NaN does: the terms decide)
+    auto reaches = [&](const float4 &s, int i) {
         const float4 b = runs[i];
-        bool on = false;
+        const float rr = s.w + kBroadMargin + b.w;
+        return !(sq3(s.x - b.x, s.y - b.y, s.z - b.z) >= rr * rr);
+    };
+    // the term of the sphere and obstacle o of run i
+    auto term = [&](const float4 &s, int i, int o) {
+        if (i < nrs) {
+            const float4 b = t.env[o];
+            const float d2 = sq3(s.x - b.x, s.y - b.y, s.z - b.z);
+            const float rr = s.w + b.w;
+            if (d2 < rr * rr) c_sph += fmaxf(0.f, rr - sqrtf(d2));
+        } else if (i < nrs + nrb) {   // inverse pose, clamp to [min, max]
+            const float4 *bx = t.env + E.ns + 5 * o;
+            const float4 mn = bx[3], mx = bx[4];
+            const float3 l = xform_rows(bx[0], bx[1], bx[2], s.x, s.y, s.z);
+            const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x);
+            const float dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y);
+            const float dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
+            const float d2 = sq3(dx, dy, dz);
+            if (d2 < s.w * s.w) c_box += s.w - sqrtf(d2);
+        } else {   // finite, local z axis
+            const float4 *cy = t.env + E.ns + 5 * E.nb + 4 * o;
+            const float4 pr = cy[3];
+            const float3 l = xform_rows(cy[0], cy[1], cy[2], s.x, s.y, s.z);
+            const float dx = sqrtf(__fmaf_rn(l.y, l.y, __fmul_rn(l.x, l.x))) - pr.x;
+            const float dz = fabsf(l.z) - pr.y;
+            const float ox = dx > 0.f ? dx : 0.f, oz = dz > 0.f ? dz : 0.f;
+            const float outside = sqrtf(__fmaf_rn(oz, oz, __fmul_rn(ox, ox)));
+            const float inside = fminf(fmaxf(dx, dz), 0.f);
+            const float pen = s.w - (outside + inside);
+            c_cyl += pen > 0.f ? pen : 0.f;
+        }
+    };
+    // first obstacle of run i within its type, and the count of the type
+    auto first = [&](int i) { return (i < nrs ? i : i < nrs + nrb ? i - nrs : i - nrs - nrb) * kWarp; };
+    auto count = [&](int i) { return i < nrs ? E.ns : i < nrs + nrb ? E.nb : E.nc; };
+
+    // --- scene: the spheres left, up to 32 at a time ---
+    for (int n0 = 0; n0 < nnear; n0 += kWarp) {
+        int at = -n0;
 #pragma unroll
         for (int m = 0; m < SPL; ++m) {
-            const float rr = cr[m] + kBroadMargin + b.w;
-            on |= !(sq3(cx[m] - b.x, cy[m] - b.y, cz[m] - b.z) >= rr * rr);   // NaN: as the terms have it
+            const int pos = at + __popc(near[m] & ((1u << lane) - 1u));
+            if ((near[m] >> lane & 1u) && pos >= 0 && pos < kWarp) w.cand[pos] = lane + kWarp * m;
+            at += __popc(near[m]);
         }
-        return __any_sync(kFull, on) != 0;
-    };
-    if (left) {
-        // --- environment spheres ---
-        const int nrs = env_clusters(E.ns), nrb = env_clusters(E.nb), nrc = env_clusters(E.nc);
+        __syncwarp();
+        const int n = min(kWarp, nnear - n0);
+        if (n >= kTogether) {   // a sphere a lane
+            const float4 s = lane < n ? w.cen[w.cand[lane]] : make_float4(kFar, kFar, kFar, 0.f);
 #pragma unroll 1
-        for (int i = 0; i < nrs; ++i) {
-            if (!reached(i)) continue;
-            const int end = min(E.ns, (i + 1) * kWarp);
+            for (int i = 0; i < nrun; ++i) {
+                if (!__any_sync(kFull, reaches(s, i))) continue;
+                const int o0 = first(i), end = min(count(i), o0 + kWarp);
 #pragma unroll 2
-            for (int o = i * kWarp; o < end; ++o) {
-                const float4 b = t.env[o];
-#pragma unroll
-                for (int m = 0; m < SPL; ++m) {
-                    if (!(left >> m & 1u)) continue;
-                    const float d2 = sq3(cx[m] - b.x, cy[m] - b.y, cz[m] - b.z);
-                    const float rr = cr[m] + b.w;
-                    if (d2 < rr * rr) c_sph += fmaxf(0.f, rr - sqrtf(d2));
+                for (int o = o0; o < end; ++o) term(s, i, o);
+            }
+        } else {   // an obstacle a lane
+            for (int x = 0; x < n; ++x) {
+                const float4 s = w.cen[w.cand[x]];
+#pragma unroll 1
+                for (int i0 = 0; i0 < nrun; i0 += kWarp) {
+                    unsigned bal = __ballot_sync(kFull, i0 + lane < nrun && reaches(s, min(i0 + lane, nrun - 1)));
+                    for (; bal; bal &= bal - 1u) {
+                        const int i = i0 + __ffs(bal) - 1, o = first(i) + lane;
+                        if (o < count(i)) term(s, i, o);
+                    }
+                    __syncwarp();
                 }
             }
         }
-        // --- cuboids (inverse pose, clamp to [min, max]) ---
-        const float4 *bx = t.env + E.ns;
-#pragma unroll 1
-        for (int i = 0; i < nrb; ++i) {
-            if (!reached(nrs + i)) continue;
-            const int end = min(E.nb, (i + 1) * kWarp);
-#pragma unroll 1
-            for (int o = i * kWarp; o < end; ++o) {
-                const float4 r0 = bx[5 * o], r1 = bx[5 * o + 1], r2 = bx[5 * o + 2], mn = bx[5 * o + 3], mx = bx[5 * o + 4];
-#pragma unroll
-                for (int m = 0; m < SPL; ++m) {
-                    if (!(left >> m & 1u)) continue;
-                    const float3 l = xform_rows(r0, r1, r2, cx[m], cy[m], cz[m]);
-                    const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x);
-                    const float dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y);
-                    const float dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
-                    const float d2 = sq3(dx, dy, dz);
-                    if (d2 < cr[m] * cr[m]) c_box += cr[m] - sqrtf(d2);
-                }
-            }
-        }
-        // --- cylinders (finite, local z axis) ---
-        const float4 *cyl = bx + 5 * E.nb;
-#pragma unroll 1
-        for (int i = 0; i < nrc; ++i) {
-            if (!reached(nrs + nrb + i)) continue;
-            const int end = min(E.nc, (i + 1) * kWarp);
-#pragma unroll 1
-            for (int o = i * kWarp; o < end; ++o) {
-                const float4 r0 = cyl[4 * o], r1 = cyl[4 * o + 1], r2 = cyl[4 * o + 2], pr = cyl[4 * o + 3];
-#pragma unroll
-                for (int m = 0; m < SPL; ++m) {
-                    if (!(left >> m & 1u)) continue;
-                    const float3 l = xform_rows(r0, r1, r2, cx[m], cy[m], cz[m]);
-                    const float dx = sqrtf(__fmaf_rn(l.y, l.y, __fmul_rn(l.x, l.x))) - pr.x;
-                    const float dz = fabsf(l.z) - pr.y;
-                    const float ox = dx > 0.f ? dx : 0.f, oz = dz > 0.f ? dz : 0.f;
-                    const float outside = sqrtf(__fmaf_rn(oz, oz, __fmul_rn(ox, ox)));
-                    const float inside = fminf(fmaxf(dx, dz), 0.f);
-                    const float pen = cr[m] - (outside + inside);
-                    c_cyl += pen > 0.f ? pen : 0.f;
-                }
-            }
-        }
+        __syncwarp();
     }
 
     // --- self collision: group pairs whose bounding spheres overlap ---
