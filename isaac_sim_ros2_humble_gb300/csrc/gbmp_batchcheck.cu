@@ -264,7 +264,8 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
             }
             ranges[nr++] = CheckRange{ti, 0, lo, std::min(lo + spb, tasks[ti].n)};
         }
-    GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, ranges_off + sizeof(CheckRange) * (size_t)nr, cudaMemcpyHostToDevice, s));
+    GBMP_CUDA(cudaMemcpyAsync(b->d_buf, b->h_buf, ranges_off + sizeof(CheckRange) * (size_t)nr,
+                              cudaMemcpyHostToDevice, s));
     GBMP_CUDA(cudaEventRecord(b->uploaded, s));
     b->pending = true;
     const auto *d_tasks = reinterpret_cast<const CheckTask *>(b->d_buf);

@@ -50,8 +50,9 @@ constexpr int kMaxGrab = 8;   // settled items taken at a time in a batch of few
 template <int K, bool CNT>
 __global__ void __launch_bounds__(kChunkWarps *kWarp, 3)
     k_edge_chunk(DevRobot R, DevEnv E, const float *__restrict__ from, const float *__restrict__ to,
-                 int *nsteps, const float *__restrict__ dir, const int *__restrict__ order, int n_edges, const EdgePlan *__restrict__ plan, unsigned long long *__restrict__ next,
-                 unsigned char *ok_out, int *first_hit_out) {
+                 int *nsteps, const float *__restrict__ dir, const int *__restrict__ order, int n_edges,
+                 const EdgePlan *__restrict__ plan, unsigned long long *__restrict__ next, unsigned char *ok_out,
+                 int *first_hit_out) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nwords = env_words(E.ns, E.nb, E.nc);
     SmemTables t = carve_tables(smem, R, nwords);

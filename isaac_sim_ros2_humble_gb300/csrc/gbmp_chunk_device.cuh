@@ -27,10 +27,11 @@
 //
 // What bounds it: instruction issue and latency, not memory (the tables live in shared
 // memory).  65,536 edges of the benchmark: 2.26 ms when every swept sphere was tested
-// against every run, 1.25 ms with the field (most chunks then have no group left).  Walking the states one after another left most lanes idle: per state of the
-// benchmark's edges 0.3 obstacle candidates and 2.3 group pairs, each pair's test a chain
-// of shared-memory loads over 7 spheres.  Side by side the chunk's 23 (state, pair) items
-// fill a warp.  And the size of the code counts: the chunk kernel's loops are not unrolled
+// against every run, 1.25 ms with the field (most chunks then have no group left).
+// Walking the states one after another left most lanes idle: per state of the benchmark's
+// edges 0.3 obstacle candidates and 2.3 group pairs, each pair's test a chain of
+// shared-memory loads over 7 spheres.  Side by side the chunk's 23 (state, pair) items fill
+// a warp (3.8 -> 2.2 ms).  And the size of the code counts: the chunk kernel's loops are not unrolled
 // (51 KB instead of 75 KB; 65,536 edges 1.21 against 1.25 ms), for the instruction cache
 // holds about one such body.
 #pragma once

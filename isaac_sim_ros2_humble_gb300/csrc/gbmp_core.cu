@@ -207,8 +207,7 @@ __global__ void k_edge_order(const int *__restrict__ nsteps, long long E, const 
 
 // Set-up, order and plan of at most kFewEdges edges by one block, a thread an edge, the
 // buckets' counts in shared memory: one launch where k_edge_setup and k_edge_order with the
-// zeroing of their counters are three (64 edges: 37 us a call, 41 with
-// the three).
+// zeroing of their counters are three (64 edges: 37 us a call, 41 with the three).
 constexpr int kFewEdges = 1024;
 __global__ void __launch_bounds__(kFewEdges)
     k_edge_few(const float *__restrict__ from, const float *__restrict__ to, int E, int L, float res, int rule,
