@@ -874,7 +874,11 @@ gbmp_status gbmp_check_states_fk(gbmp_robot r, gbmp_env env, const float *d_q, i
             int grid = 0;
             st = persistent_grid(k_check_costs<SPL>, smem, r->num_sms, &grid);
             if (st) return st;
-            if (need < grid) grid = (int)need;
+            // three times the blocks that are resident: a state in clutter costs ten times a
+            // free one, and the blocks that follow even that out (20,011 states: 165 us with
+            // as many as are resident, 162 with twice, 145 with three times, 153 with a block
+            // for every eight states, which stages the tables for each)
+            grid = (int)std::min<long long>(need, 3LL * grid);
             ProfScope ps(GBMP_PROF_CHECK_STATES, s);
             k_check_costs<SPL><<<grid, kWarpsPerBlock * kWarp, smem, s>>>(D, E, d_q, n, d_verdict, d_costs, d_total,
                                                                           d_poses, d_centers);

@@ -785,7 +785,8 @@ __device__ inline bool warp_collide_culled(const SmemTables &t, const DevRobot &
 // after another against an obstacle a lane.  Summing all pairs (336 obstacles x 110 spheres
 // and 3,192 self pairs a state) took 628 us for 20,011 states; each lane's own four spheres
 // with this culling 225 us; listed 165 us (172 when a sphere always has a lane, 287 when it
-// never has; lists of 5 or 16 as the line between the two: 166).
+// never has; lists of 5 or 16 as the line between the two: 166), and 145 us with the blocks
+// that its launch takes since.
 constexpr int kTogether = 10;
 template <int SPL>
 __device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
