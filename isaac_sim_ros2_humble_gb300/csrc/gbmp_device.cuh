@@ -123,6 +123,14 @@ struct DevEnv {
 constexpr int kFieldCells = 32;
 constexpr double kFieldBorder = 0.2;     // metres of field around the obstacles
 constexpr double kFieldLargest = 1.0;    // bounding radius of the obstacles that span the field
+// Share of the lengths behind a stored distance that it is reduced by, for rounding: with
+// unit roundoff u = 2^-24, cell centre c, obstacle distance d and `size` (a sphere's radius,
+// the translation of an inverse pose) the distance is off by at most 8 u (d + |c| + size),
+// the way to a query by 4 u way, and the exact test of the query by 8 u (|c| + 1.8 way +
+// size); where they decide, way <= d, so 27 u (d + |c| + size) covers them.  A few micrometres in a
+// scene of some metres.  Without it a scene that held one obstacle 600 km away, in cells 19
+// km wide, cleared spheres that were 0.8 mm inside an obstacle next to the robot.
+constexpr float kFieldSlack = 2e-6f;     // 33 u
 constexpr int kFlField = 24;             // box distance, cell and bound of one lookup
 
 __host__ __device__ inline int env_clusters(int n) { return (n + 31) / 32; }
@@ -428,28 +436,32 @@ __device__ __forceinline__ float sq3(float dx, float dy, float dz) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
-// True when no obstacle of the scene comes within `rad` of (x, y, z): the sphere lies
-// outside the box of all obstacles, or the distance stored for the nearest cell centre,
-// less the way there (distances change by no more than the way), exceeds rad.  False says
-// nothing.  One load (L1 or L2: a field is 512 KB at most) in place of a test
-// against every obstacle; with the cells of a 2 m scene 6 cm wide the bound is 3 cm short on
-// average.
-// Callers' radii carry kBroadMargin, which covers the rounding here and in the exact tests.
 // Outside the box of all obstacles, by more than rad.
 __device__ __forceinline__ bool scene_outside(const DevEnv &E, float x, float y, float z, float rad) {
     const float ax = fmaxf(fmaxf(E.lox - x, x - E.hix), 0.f), ay = fmaxf(fmaxf(E.loy - y, y - E.hiy), 0.f),
                 az = fmaxf(fmaxf(E.loz - z, z - E.hiz), 0.f);
     return ax * ax + ay * ay + az * az > rad * rad;
 }
+// Centre of cell i along an axis of the field, rounded the same wherever it is used.
+__device__ __forceinline__ float cell_centre(float origin, float h, int i) {
+    return __fmaf_rn((float)i + 0.5f, h, origin);
+}
 // The cell nearest to (x, y, z) and the way to its centre.
 __device__ __forceinline__ const float4 *scene_cell(const DevEnv &E, float x, float y, float z, float &way) {
     const int ix = min(max((int)((x - E.ox) * E.inv_h), 0), E.nx - 1), iy = min(max((int)((y - E.oy) * E.inv_h), 0), E.ny - 1),
               iz = min(max((int)((z - E.oz) * E.inv_h), 0), E.nz - 1);
-    const float dx = x - (E.ox + ((float)ix + 0.5f) * E.h), dy = y - (E.oy + ((float)iy + 0.5f) * E.h),
-                dz = z - (E.oz + ((float)iz + 0.5f) * E.h);
+    const float dx = x - cell_centre(E.ox, E.h, ix), dy = y - cell_centre(E.oy, E.h, iy), dz = z - cell_centre(E.oz, E.h, iz);
     way = sqrtf(dx * dx + dy * dy + dz * dz);
     return E.field + ((iz * E.ny + iy) * E.nx + ix);
 }
+// True when no obstacle of the scene comes within `rad` of (x, y, z): the sphere lies
+// outside the box of all obstacles, or the distance stored for the nearest cell centre,
+// less the way there (distances change by no more than the way), exceeds rad.  False says
+// nothing.  One load (L1 or L2: a field is 512 KB at most) in place of a test
+// against every obstacle; with the cells of a 2 m scene 6 cm wide the bound is 3 cm short on
+// average.
+// The stored distances are short by what rounding can take (kFieldSlack); the radii of the
+// callers carry kBroadMargin on top.
 __device__ __forceinline__ bool scene_far(const DevEnv &E, float x, float y, float z, float rad) {
     if (!E.field) return E.ns + E.nb + E.nc == 0;
     if (scene_outside(E, x, y, z, rad)) return true;

@@ -8,7 +8,7 @@ namespace gbmp {
 
 // The three least distances from every cell's centre to an obstacle (spheres |c - o| - r,
 // cuboids the distance to the box, cylinders the signed distance) and the obstacles of the
-// first two: eight lanes a cell, each an eighth of the obstacles, then merged (one lane a
+// first two, every distance short by kFieldSlack of what it was made from: eight lanes a cell, each an eighth of the obstacles, then merged (one lane a
 // cell leaves 32,768 threads with a chain over every obstacle: a scene of 336 took 75 us
 // longer to create, 45 us with eight).
 constexpr int kFieldLanes = 8;
@@ -34,32 +34,36 @@ __global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float4 *__restric
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, cell = tid / kFieldLanes, o0 = tid % kFieldLanes;
     const bool in = cell < E.nx * E.ny * E.nz;
     const int ix = cell % E.nx, iy = cell / E.nx % E.ny, iz = cell / (E.nx * E.ny);
-    const float x = E.ox + ((float)ix + 0.5f) * E.h, y = E.oy + ((float)iy + 0.5f) * E.h,
-                z = E.oz + ((float)iz + 0.5f) * E.h;
+    const float x = cell_centre(E.ox, E.h, ix), y = cell_centre(E.oy, E.h, iy), z = cell_centre(E.oz, E.h, iz);
+    const float c1 = fabsf(x) + fabsf(y) + fabsf(z);
+    auto least = [&](float d, float size) { return d - kFieldSlack * (fabsf(d) + c1 + size); };
     Nearest3 n;
     const float4 *w = E.words;
 #pragma unroll 4
     for (int o = o0; o < E.ns; o += kFieldLanes) {
         const float4 b = __ldg(w + o);
-        n.add(sqrtf(sq3(x - b.x, y - b.y, z - b.z)) - b.w, o);
+        n.add(least(sqrtf(sq3(x - b.x, y - b.y, z - b.z)) - b.w, fabsf(b.w)), o);
     }
     w += E.ns;
 #pragma unroll 2
     for (int o = o0; o < E.nb; o += kFieldLanes) {
         const float4 mn = __ldg(w + 5 * o + 3), mx = __ldg(w + 5 * o + 4);
-        const float3 l = xform_rows(__ldg(w + 5 * o), __ldg(w + 5 * o + 1), __ldg(w + 5 * o + 2), x, y, z);
+        const float4 r0 = __ldg(w + 5 * o), r1 = __ldg(w + 5 * o + 1), r2 = __ldg(w + 5 * o + 2);
+        const float3 l = xform_rows(r0, r1, r2, x, y, z);
         const float dx = l.x - fminf(fmaxf(l.x, mn.x), mx.x), dy = l.y - fminf(fmaxf(l.y, mn.y), mx.y),
                     dz = l.z - fminf(fmaxf(l.z, mn.z), mx.z);
-        n.add(sqrtf(sq3(dx, dy, dz)), E.ns + o);
+        n.add(least(sqrtf(sq3(dx, dy, dz)), fabsf(r0.w) + fabsf(r1.w) + fabsf(r2.w)), E.ns + o);
     }
     w += 5 * E.nb;
 #pragma unroll 2
     for (int o = o0; o < E.nc; o += kFieldLanes) {
         const float4 pr = __ldg(w + 4 * o + 3);
-        const float3 l = xform_rows(__ldg(w + 4 * o), __ldg(w + 4 * o + 1), __ldg(w + 4 * o + 2), x, y, z);
+        const float4 r0 = __ldg(w + 4 * o), r1 = __ldg(w + 4 * o + 1), r2 = __ldg(w + 4 * o + 2);
+        const float3 l = xform_rows(r0, r1, r2, x, y, z);
         const float dx = sqrtf(l.x * l.x + l.y * l.y) - pr.x, dz = fabsf(l.z) - pr.y;
         const float ox = fmaxf(dx, 0.f), oz = fmaxf(dz, 0.f);
-        n.add(sqrtf(ox * ox + oz * oz) + fminf(fmaxf(dx, dz), 0.f), E.ns + E.nb + o);
+        n.add(least(sqrtf(ox * ox + oz * oz) + fminf(fmaxf(dx, dz), 0.f), fabsf(r0.w) + fabsf(r1.w) + fabsf(r2.w)),
+              E.ns + E.nb + o);
     }
 #pragma unroll
     for (int off = 1; off < kFieldLanes; off <<= 1) {
