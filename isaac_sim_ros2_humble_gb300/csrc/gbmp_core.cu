@@ -721,6 +721,18 @@ static void cluster_spheres(const std::vector<double> &c, const std::vector<doub
     }
 }
 
+// How far the rows of a rotation are from orthonormal (NaN where an entry is not finite).
+static double rotation_error(const float *R) {
+    double worst = 0.0;
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j <= i; ++j) {
+            double d = i == j ? -1.0 : 0.0;
+            for (int a = 0; a < 3; ++a) d += (double)R[3 * i + a] * R[3 * j + a];
+            if (!(std::fabs(d) <= worst)) worst = std::isnan(worst) ? worst : std::fabs(d);
+        }
+    return worst;
+}
+
 gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_t nb, const float *bp,
                             const float *brot, const float *bmin, const float *bmax, int32_t nc, const float *cp,
                             const float *crot, const float *crad, const float *chei, gbmp_env *out) {
@@ -742,6 +754,16 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
         for (int a = 0; a < 3; ++a) sc[3 * i + a] = sp[3 * i + a];
         srd[i] = sr[i];
     }
+    // Bounding spheres hold for rotations: with rows off orthonormal by e an obstacle reaches
+    // 6 e of its size farther at most.  Up to half of kBroadMargin, which the tests that use
+    // the spheres add, is let pass; more, or a number that is not finite, makes the scene loose.
+    double skew = 0.0;
+    bool loose = false;
+    auto bounded = [&](const float *pos, const float *rot, double size) {
+        const double e = rotation_error(rot);
+        loose = loose || !(6.0 * e * size <= 0.5 * kBroadMargin) || !std::isfinite(pos[0] + pos[1] + pos[2]);
+        skew = std::max(skew, e);
+    };
     for (int i = 0; i < nb; ++i) {   // box: centre pos + R (min + max) / 2, radius half the diagonal
         const float *R = brot + 9 * i;
         double l[3], h2 = 0.0;
@@ -753,10 +775,12 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
         for (int a = 0; a < 3; ++a)
             bc[3 * i + a] = bp[3 * i + a] + R[3 * a] * l[0] + R[3 * a + 1] * l[1] + R[3 * a + 2] * l[2];
         brd[i] = std::sqrt(h2);
+        bounded(bp + 3 * i, R, brd[i] + std::sqrt(l[0] * l[0] + l[1] * l[1] + l[2] * l[2]));
     }
     for (int i = 0; i < nc; ++i) {   // cylinder: centre pos, radius sqrt(r^2 + (h/2)^2)
         for (int a = 0; a < 3; ++a) cc[3 * i + a] = cp[3 * i + a];
         crd[i] = std::sqrt((double)crad[i] * crad[i] + 0.25 * (double)chei[i] * chei[i]);
+        bounded(cp + 3 * i, crot + 9 * i, crd[i]);
     }
     std::vector<int> os(ns), ob(nb), oc(nc);
     for (int i = 0; i < ns; ++i) os[i] = i;
@@ -808,14 +832,15 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     bound(sc, srd);
     bound(bc, brd);
     bound(cc, crd);
-    const bool field = scene_field_plan(bounds, E);
+    E.loose = loose;
+    const bool field = !loose && scene_field_plan(bounds, E);
     const size_t wbytes = sizeof(float4) * e->h_words.size();
     cudaError_t err = cudaMalloc(&e->d_words, wbytes + (field ? sizeof(float4) * (size_t)E.nx * E.ny * E.nz : 0));
     if (err == cudaSuccess) err = cudaMemcpy(e->d_words, e->h_words.data(), wbytes, cudaMemcpyHostToDevice);
     E.words = e->d_words;
     if (err == cudaSuccess && field) {
         float4 *values = e->d_words + e->h_words.size();
-        err = scene_field_build(E, values, nullptr);
+        err = scene_field_build(E, kFieldSlack + (float)(6.0 * skew), values, nullptr);
         if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
         E.field = values;
     }

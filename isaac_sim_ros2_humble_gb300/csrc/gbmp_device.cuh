@@ -115,6 +115,10 @@ struct DevEnv {
     int nx, ny, nz;
     float ox, oy, oz, h, inv_h;
     float lox, loy, loz, hix, hiy, hiz;
+    // 1: an obstacle may reach beyond its bounding sphere (an unbounded box, a rotation that
+    // is none).  The scene then has no field, and state checks and plans of one problem pass over no
+    // run of obstacles.
+    int loose;
 };
 
 // Cells along the field's longest side (512 KB a scene at most).  65,536 edges of the 8-DOF
@@ -832,7 +836,7 @@ __device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const 
     auto reaches = [&](const float4 &s, int i) {
         const float4 b = runs[i];
         const float rr = s.w + kBroadMargin + b.w;
-        return !(sq3(s.x - b.x, s.y - b.y, s.z - b.z) >= rr * rr);
+        return E.loose || !(sq3(s.x - b.x, s.y - b.y, s.z - b.z) >= rr * rr);
     };
     // the term of the sphere and obstacle o of run i
     auto term = [&](const float4 &s, int i, int o) {

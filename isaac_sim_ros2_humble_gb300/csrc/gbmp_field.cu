@@ -8,7 +8,8 @@ namespace gbmp {
 
 // The three least distances from every cell's centre to an obstacle (spheres |c - o| - r,
 // cuboids the distance to the box, cylinders the signed distance) and the obstacles of the
-// first two, every distance short by kFieldSlack of what it was made from: eight lanes a cell, each an eighth of the obstacles, then merged (one lane a
+// first two, every distance short by `slack` of what it was made from (kFieldSlack, and what
+// rotations that are not quite orthonormal change distances by): eight lanes a cell, each an eighth of the obstacles, then merged (one lane a
 // cell leaves 32,768 threads with a chain over every obstacle: a scene of 336 took 75 us
 // longer to create, 45 us with eight).
 constexpr int kFieldLanes = 8;
@@ -30,13 +31,13 @@ struct Nearest3 {
     }
 };
 
-__global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float4 *__restrict__ field) {
+__global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float slack, float4 *__restrict__ field) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, cell = tid / kFieldLanes, o0 = tid % kFieldLanes;
     const bool in = cell < E.nx * E.ny * E.nz;
     const int ix = cell % E.nx, iy = cell / E.nx % E.ny, iz = cell / (E.nx * E.ny);
     const float x = cell_centre(E.ox, E.h, ix), y = cell_centre(E.oy, E.h, iy), z = cell_centre(E.oz, E.h, iz);
     const float c1 = fabsf(x) + fabsf(y) + fabsf(z);
-    auto least = [&](float d, float size) { return d - kFieldSlack * (fabsf(d) + c1 + size); };
+    auto least = [&](float d, float size) { return d - slack * (fabsf(d) + c1 + size); };
     Nearest3 n;
     const float4 *w = E.words;
 #pragma unroll 4
@@ -121,9 +122,9 @@ bool scene_field_plan(const std::vector<double> &b, DevEnv &E) {
     return true;
 }
 
-cudaError_t scene_field_build(const DevEnv &E, float4 *field, cudaStream_t s) {
+cudaError_t scene_field_build(const DevEnv &E, float slack, float4 *field, cudaStream_t s) {
     const int cells = E.nx * E.ny * E.nz;
-    k_scene_field<<<(cells * kFieldLanes + 255) / 256, 256, 0, s>>>(E, field);
+    k_scene_field<<<(cells * kFieldLanes + 255) / 256, 256, 0, s>>>(E, slack, field);
     return cudaGetLastError();
 }
 

@@ -198,9 +198,10 @@ gbmp_status edge_chunk_launch(const DevRobot &R, const DevEnv &E, int K, int gri
 
 namespace gbmp {
 // Distance field of a scene (gbmp_field.cu): region and cells from the bounding spheres
-// (4 doubles each), then the values, written to `field` on stream s.
+// (4 doubles each), then the values, short by `slack` of their lengths, written to `field`
+// on stream s.
 bool scene_field_plan(const std::vector<double> &bounds, DevEnv &E);
-cudaError_t scene_field_build(const DevEnv &E, float4 *field, cudaStream_t s);
+cudaError_t scene_field_build(const DevEnv &E, float slack, float4 *field, cudaStream_t s);
 }  // namespace gbmp
 
 struct gbmp_env_s {

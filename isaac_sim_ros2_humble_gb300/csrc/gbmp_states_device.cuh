@@ -108,7 +108,7 @@ __device__ __forceinline__ bool warp_sphere_hits(const SmemTables &t, const DevE
         if (c0 + lane < nrun) {
             const float4 b = runs[c0 + lane];
             const float rr = r + kBroadMargin + b.w;
-            on = !(sq3(c.x - b.x, c.y - b.y, c.z - b.z) >= rr * rr);   // NaN: as the tests below have it
+            on = E.loose || !(sq3(c.x - b.x, c.y - b.y, c.z - b.z) >= rr * rr);   // NaN: as the tests below have it
         }
         unsigned bal = __ballot_sync(kFull, on);
         if (CNT) fl += (unsigned long long)min(kWarp, nrun - c0) * kFlGroupPair + (unsigned long long)__popc(bal) * kWarp * kFlSphereX;
