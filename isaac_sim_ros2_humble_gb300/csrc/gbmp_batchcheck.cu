@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
 
 // `ks` states a warp at a time.  256 requests over 4 robots and 16 scenes, 1.57 million
 // states: 5.38 ms with one warp for each state, 1.53 ms now.
-template <bool CNT>
+template <bool CNT, bool TIGHT>
 __global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStatesWarps)
     k_batch_verdicts(const CheckTask *__restrict__ tasks, const CheckRange *__restrict__ ranges, int ks) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStates
     const StatesScratch sc = carve_states(smem + smem_tables_bytes(R, nwords), R, ks, warp);
     const int vec = (reinterpret_cast<unsigned long long>(sT.poses) & 15ull) == 0;
     for (long long s = sB.lo + warp * ks; s < sB.hi; s += warps * ks)
-        check_verdicts<CNT>(t, R, E, sc, sT.q, s, (int)min((long long)ks, sB.hi - s), sT.verdict, sT.poses, sT.centers,
-                            vec, lane);
+        check_verdicts<CNT, TIGHT>(t, R, E, sc, sT.q, s, (int)min((long long)ks, sB.hi - s), sT.verdict, sT.poses,
+                                   sT.centers, vec, lane);
 }
 
 #define GBMP_BATCH_SPL_SWITCH(spl, ...)                    \
@@ -192,6 +192,7 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
     size_t smem = 0;   // of the costs' kernel, which also says which requests fit
     size_t tables = 0;
     DevRobot widest{};
+    bool tight = true;   // every scene is
     long long total = 0;
     unsigned long long *work = work_counter();
     for (int i : b->order) {
@@ -199,7 +200,7 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         CheckTask &T = tasks[nt++];
         T.R = cost ? q.robot->dev : q.robot->dev_chunk;
         T.R.work = work;
-        T.E = q.env->dev();
+        T.E = q.env->dev_states();
         T.q = q.d_q;
         T.n = q.n;
         T.verdict = q.d_verdict;
@@ -213,6 +214,7 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         tables = std::max(tables, smem_tables_bytes(T.R, words));
         widest.L = std::max(widest.L, T.R.L);
         widest.G = std::max(widest.G, T.R.G);
+        tight = tight && q.env->tight;
         total += q.n;
     }
     if (nt == 0) return GBMP_OK;
@@ -228,7 +230,8 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
     if (cost) {
         GBMP_BATCH_SPL_SWITCH(spl, { fn = (const void *)k_batch_costs<SPL>; });
     } else {
-        fn = work ? (const void *)k_batch_verdicts<true> : (const void *)k_batch_verdicts<false>;
+        fn = work ? (tight ? (const void *)k_batch_verdicts<true, true> : (const void *)k_batch_verdicts<true, false>)
+                  : (tight ? (const void *)k_batch_verdicts<false, true> : (const void *)k_batch_verdicts<false, false>);
     }
     gbmp_status st = ensure_smem_optin(fn);
     if (st) return st;

@@ -115,10 +115,6 @@ struct DevEnv {
     int nx, ny, nz;
     float ox, oy, oz, h, inv_h;
     float lox, loy, loz, hix, hiy, hiz;
-    // 1: an obstacle may reach beyond its bounding sphere (an unbounded box, a rotation that
-    // is none).  The scene then has no field, and state checks and plans of one problem pass over no
-    // run of obstacles.
-    int loose;
 };
 
 // Cells along the field's longest side (512 KB a scene at most).  65,536 edges of the 8-DOF
@@ -127,6 +123,7 @@ struct DevEnv {
 constexpr int kFieldCells = 32;
 constexpr double kFieldBorder = 0.2;     // metres of field around the obstacles
 constexpr double kFieldLargest = 1.0;    // bounding radius of the obstacles that span the field
+constexpr double kFieldFine = 0.1;       // metres, cells of a tight scene
 // Share of the lengths behind a stored distance that it is reduced by, for rounding: with
 // unit roundoff u = 2^-24, cell centre c, obstacle distance d and `size` (a sphere's radius,
 // the translation of an inverse pose) the distance is off by at most 8 u (d + |c| + size),
@@ -836,7 +833,7 @@ __device__ inline void warp_costs(const SmemTables &t, const DevRobot &R, const 
     auto reaches = [&](const float4 &s, int i) {
         const float4 b = runs[i];
         const float rr = s.w + kBroadMargin + b.w;
-        return E.loose || !(sq3(s.x - b.x, s.y - b.y, s.z - b.z) >= rr * rr);
+        return !(sq3(s.x - b.x, s.y - b.y, s.z - b.z) >= rr * rr);
     };
     // the term of the sphere and obstacle o of run i
     auto term = [&](const float4 &s, int i, int o) {
@@ -966,6 +963,21 @@ __device__ inline void store_fk(const SmemTables &t, const DevRobot &R, const Wa
             C[3 * k] = p.x; C[3 * k + 1] = p.y; C[3 * k + 2] = p.z;
         }
     }
+}
+
+// State s of a verdict check in a scene without a field, one warp: every obstacle against
+// every group sphere.
+template <int SPL>
+__device__ inline void check_each(const SmemTables &t, const DevRobot &R, const DevEnv &E, const WarpScratch &w,
+                                  const float *__restrict__ q, long long s, unsigned char *__restrict__ verdict,
+                                  float *__restrict__ poses, float *__restrict__ centers, int lane) {
+    for (int j = lane; j < R.L; j += kWarp) w.q[j] = q[s * R.L + j];
+    __syncwarp();
+    warp_fk(t, R.L, w, lane);
+    if (poses || centers) store_fk(t, R, w, s, poses, centers, lane);
+    const bool hit = R.cull ? warp_collide_culled<SPL>(t, R, E, w, lane) : warp_collide<SPL>(t, R, E, w, lane);
+    if (verdict && lane == 0) verdict[s] = hit;
+    __syncwarp();
 }
 
 // State s of a cost check, one warp: FK of state s of q, its poses / centres when asked for,

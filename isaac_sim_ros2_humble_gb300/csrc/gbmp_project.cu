@@ -391,7 +391,7 @@ __device__ __forceinline__ bool recorded_pass(const SmemTables &t, const DevRobo
         }
     }
     if (__any_sync(kFull, bad)) return false;
-    return warp_verdicts<false>(t, R, E, w.sc, nb, lane) == 0u;
+    return warp_verdicts<false, false>(t, R, E, w.sc, nb, lane) == 0u;
 }
 
 template <int U>
@@ -708,7 +708,7 @@ extern "C" gbmp_status gbmp_constrained_motions(gbmp_robot r, gbmp_env env, cons
         p.reference[k] = proj->reference[k];
         p.tolerance[k] = proj->tolerance[k];
     }
-    const DevEnv E = env->dev();
+    const DevEnv E = env->dev_states();
     DevRobot D = r->dev_chunk;
     D.work = nullptr;
     const int nwords = env_words(E.ns, E.nb, E.nc);

@@ -338,7 +338,7 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     // next to the scene: faster at every lane count (the shelf at range 0.5: 1 lane 908 ->
     // 530 us, 32 lanes 294 -> 156, 1,024 lanes 345 -> 163; at range 0.1: 2.45 -> 2.39 ms,
     // 0.55 -> 0.52, 0.87 -> 0.65).  Chunks pass over runs of obstacles, so not in a loose scene
-    const bool chunk = r->dev_chunk.cull && !E.loose && rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk) <= kSmemLimit;
+    const bool chunk = r->dev_chunk.cull && !env->loose && rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk) <= kSmemLimit;
     DevRobot DR = chunk ? r->dev_chunk : r->dev;
     DR.work = nullptr;
     const size_t smem = rrtc_block_smem(DR, nwords, chunk ? kRrtcSoloChunk : 0);
