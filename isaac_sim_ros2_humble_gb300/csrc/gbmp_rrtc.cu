@@ -335,10 +335,14 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     const DevEnv E = env->dev();
     const int nwords = env_words(E.ns, E.nb, E.nc);
     // by chunks of states where the tables allow it (at most 32 groups) and the scratch fits
-    // next to the scene: faster at every lane count (the shelf at range 0.5: 1 lane 908 ->
-    // 530 us, 32 lanes 294 -> 156, 1,024 lanes 345 -> 163; at range 0.1: 2.45 -> 2.39 ms,
-    // 0.55 -> 0.52, 0.87 -> 0.65).  Chunks pass over runs of obstacles, so not in a loose scene
-    const bool chunk = r->dev_chunk.cull && !env->loose && rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk) <= kSmemLimit;
+    // next to the scene: faster at every lane count, with a path and without (p50 of 48
+    // problems on the shelf, range 0.1: 1 lane 2.44 -> 1.83 ms, 64 lanes 0.51 -> 0.35, 456
+    // lanes 0.55 -> 0.41, 1,024 lanes 0.68 -> 0.45; problems of the uneven mix without a path:
+    // 64 lanes 620 -> 415 ms, 1,024 lanes 68 -> 53 ms).  Chunks pass over runs of obstacles, so
+    // not in a loose scene
+    const bool chunk = r->dev_chunk.cull && !env->loose &&
+                       std::max(rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk), rrtc_block_smem(r->dev, nwords, 0)) <=
+                           kSmemLimit;
     DevRobot DR = chunk ? r->dev_chunk : r->dev;
     DR.work = nullptr;
     const size_t smem = rrtc_block_smem(DR, nwords, chunk ? kRrtcSoloChunk : 0);
@@ -462,7 +466,7 @@ struct gbmp_batch_planner_s {
 };
 
 static gbmp_status batch_launch(gbmp_batch_planner b, int n, int lpp, const RrtcParams &prm, int spl, bool cull,
-                                size_t smem, double limit_s, cudaStream_t st) {
+                                size_t smem, size_t reserve, double limit_s, cudaStream_t st) {
     GBMP_CUDA(cudaMemcpyAsync(b->d_table, b->h_table, sizeof(BatchProblem) * n, cudaMemcpyHostToDevice, st));
     GBMP_CUDA(cudaMemcpyAsync(b->d_roots, b->h_roots, sizeof(float) * (size_t)n * 2 * b->max_links,
                               cudaMemcpyHostToDevice, st));
@@ -476,8 +480,10 @@ static gbmp_status batch_launch(gbmp_batch_planner b, int n, int lpp, const Rrtc
     {
         ProfScope ps(GBMP_PROF_OTHER, st);
         int *rr = (int *)(b->d_deadline + 1);
-        const cudaError_t ce = spl <= 4 ? rrtc_batch_launch_lo(spl, cull, n * lpp, smem, st, b->d_table, n, lpp, prm, rr)
-                                        : rrtc_batch_launch_hi(spl, cull, n * lpp, smem, st, b->d_table, n, lpp, prm, rr);
+        const cudaError_t ce =
+            cull       ? rrtc_batch_launch_chunk(n * lpp, smem, reserve, st, b->d_table, n, lpp, prm, rr)
+            : spl <= 4 ? rrtc_batch_launch_lo(spl, n * lpp, smem, reserve, st, b->d_table, n, lpp, prm, rr)
+                       : rrtc_batch_launch_hi(spl, n * lpp, smem, reserve, st, b->d_table, n, lpp, prm, rr);
         if (ce != cudaSuccess) {
             set_error("planning kernel launch (%zu bytes of shared memory): %s", smem, cudaGetErrorString(ce));
             stt = ce == cudaErrorInvalidValue ? GBMP_ERR_CAPACITY : GBMP_ERR_CUDA;
@@ -690,7 +696,9 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
                    "unknown step rule or resolution out of range");
     int spl = 1;
     bool cull = true;
-    size_t smem = 0;
+    // Shared memory of the two forms of the edge checks, and what a problem may need: the room
+    // for both scratches decides which scenes are accepted.
+    size_t smem_chunk = 0, smem_state = 0, reserve = 0;
     auto *pool = static_cast<unsigned char *>(b->pool);
     const size_t nodes_b = align16(sizeof(float) * (size_t)b->cap * b->stride);
     const size_t par_b = align16(sizeof(int) * (size_t)b->cap);
@@ -704,7 +712,10 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
         const DevEnv E = pr.env->dev();
         spl = std::max(spl, R.spl);
         cull = cull && R.cull;
-        smem = std::max(smem, rrtc_block_smem(R, env_words(E.ns, E.nb, E.nc), kRrtcChunk));
+        const int nwords = env_words(E.ns, E.nb, E.nc);
+        smem_chunk = std::max(smem_chunk, rrtc_block_smem(R, nwords, kRrtcChunk));
+        smem_state = std::max(smem_state, rrtc_block_smem(R, nwords, 0));
+        reserve = std::max(reserve, rrtc_block_smem(R, nwords, 0) + (R.cull ? smem_chunk_bytes(R, kRrtcChunk) * kRrtcWarps : 0));
         BatchProblem &bp = b->h_table[i];
         bp.R = R;
         bp.R.work = nullptr;
@@ -739,6 +750,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
         }
         b->h_flags[i] = 0;
     }
+    const size_t smem = cull ? smem_chunk : smem_state;   // by chunks where every robot can
     RrtcParams prm;
     prm.lanes = lanes_per_problem;
     prm.max_iters = s->max_iters;
@@ -781,7 +793,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
             cudaStream_t cap_st;
             GBMP_CUDA(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking));
             GBMP_CUDA(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
-            gbmp_status bs = batch_launch(b, n, lanes_per_problem, prm, spl, cull, smem, lim, cap_st);
+            gbmp_status bs = batch_launch(b, n, lanes_per_problem, prm, spl, cull, smem, reserve, lim, cap_st);
             cudaGraph_t g = nullptr;
             cudaError_t ce = cudaStreamEndCapture(cap_st, &g);
             cudaStreamDestroy(cap_st);
@@ -799,7 +811,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
         count_launch(4);
         GBMP_CUDA(cudaGraphLaunch(exec, st));
     } else {
-        gbmp_status bs = batch_launch(b, n, lanes_per_problem, prm, spl, cull, smem, lim, st);
+        gbmp_status bs = batch_launch(b, n, lanes_per_problem, prm, spl, cull, smem, reserve, lim, st);
         if (bs) return bs;
     }
     GBMP_CUDA(cudaEventRecord(b->ev1, st));

@@ -18,13 +18,15 @@ constexpr int kRrtcThreads = kRrtcWarps * kWarp;
 constexpr int kRrtcChunk = 4;
 constexpr int kRrtcSoloChunk = 8;
 
-// Shared memory of a planning block: staged tables, four warp scratches, the lane's
-// joint vectors and flags, and, when the edge checks run by chunks of `chunk` states
-// (robots of at most 32 sphere groups), four chunk scratches.
+// Shared memory of a planning block: staged tables, the lane's joint vectors and flags, and
+// four scratches: of chunks of `chunk` states where the edge checks run by chunks (robots of at
+// most 32 sphere groups), else of a state.  (While the chunk forms held both, three blocks
+// of the single-problem kernel fitted on an SM instead of four, and ten problems without a path took 71 ms
+// at 1,024 lanes; 53 ms now, 67 with k_rrtc.)
 __host__ __device__ inline size_t rrtc_misc_bytes() { return align16(6 * kMaxLinks * 4 + 256); }
 __host__ __device__ inline size_t rrtc_block_smem(const DevRobot &R, int nwords, int chunk) {
-    return smem_tables_bytes(R, nwords) + smem_warp_bytes(R) * kRrtcWarps + rrtc_misc_bytes() +
-           (chunk && R.cull ? smem_chunk_bytes(R, chunk) * kRrtcWarps : 0);
+    return smem_tables_bytes(R, nwords) + rrtc_misc_bytes() +
+           (chunk ? smem_chunk_bytes(R, chunk) : smem_warp_bytes(R)) * kRrtcWarps;
 }
 
 enum : int { kStRunning = 0, kStSolved = 1, kStNodeCap = 2, kStIterCap = 3, kStDeadline = 4 };
@@ -106,19 +108,22 @@ struct BatchProblem {
 };
 
 // Launchers of the planning kernels, defined by the instantiation units: *_lo for 1 to 4
-// spheres per lane, *_hi for 5 to 8.  Each sets the kernel's dynamic shared-memory limit
-// to `smem` and launches `grid` blocks of kRrtcThreads on `st`; the CUDA error of either
-// step is returned.
+// spheres per lane, *_hi for 5 to 8, *_chunk for any (edge checks by chunks).  Each raises the
+// kernel's dynamic shared-memory limit to `smem` (batched: to `reserve`, at least as much)
+// where it is lower (a captured launch of more may be replayed later) and launches `grid`
+// blocks of kRrtcThreads on `st`; the CUDA error of either step is returned.
 cudaError_t rrtc_launch_lo(int spl, bool cull, int grid, size_t smem, cudaStream_t st, const DevRobot &R,
                            const DevEnv &E, const RrtcDev &P, const RrtcParams &prm);
 cudaError_t rrtc_launch_hi(int spl, bool cull, int grid, size_t smem, cudaStream_t st, const DevRobot &R,
                            const DevEnv &E, const RrtcDev &P, const RrtcParams &prm);
 cudaError_t rrtc_launch_chunk(int grid, size_t smem, cudaStream_t st, const DevRobot &R, const DevEnv &E,
                             const RrtcDev &P, const RrtcParams &prm);
-cudaError_t rrtc_batch_launch_lo(int spl, bool cull, int grid, size_t smem, cudaStream_t st,
+cudaError_t rrtc_batch_launch_chunk(int grid, size_t smem, size_t reserve, cudaStream_t st, const BatchProblem *probs,
+                                    int n, int lanes_per_problem, const RrtcParams &prm, int *rr);
+cudaError_t rrtc_batch_launch_lo(int spl, int grid, size_t smem, size_t reserve, cudaStream_t st,
                                  const BatchProblem *probs, int n, int lanes_per_problem, const RrtcParams &prm,
                                  int *rr);
-cudaError_t rrtc_batch_launch_hi(int spl, bool cull, int grid, size_t smem, cudaStream_t st,
+cudaError_t rrtc_batch_launch_hi(int spl, int grid, size_t smem, size_t reserve, cudaStream_t st,
                                  const BatchProblem *probs, int n, int lanes_per_problem, const RrtcParams &prm,
                                  int *rr);
 

@@ -280,8 +280,15 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
     SmemTables t = carve_tables(smem, R, nwords);
     if (!stage_tables(R, E, t, nwords)) return;
     unsigned char *p = smem + smem_tables_bytes(R, nwords);
-    WarpScratch w = carve_warp(p, R, threadIdx.x / kWarp);
-    p += smem_warp_bytes(R) * kRrtcWarps;
+    WarpScratch w{};
+    ChunkScratch cs{};
+    if constexpr (CULL && CHUNK > 0) {
+        carve_chunk(p, R, CHUNK, threadIdx.x / kWarp, cs);
+        p += smem_chunk_bytes(R, CHUNK) * kRrtcWarps;
+    } else {
+        w = carve_warp(p, R, threadIdx.x / kWarp);
+        p += smem_warp_bytes(R) * kRrtcWarps;
+    }
     float *q_s = reinterpret_cast<float *>(p);          // sample / steered node
     float *q_a = q_s + kMaxLinks;                        // nearest node / current node
     float *q_b = q_a + kMaxLinks;                        // connect target
@@ -291,8 +298,6 @@ __device__ void rrtc_lane(const DevRobot &R, const DevEnv &E, const RrtcDev &P, 
     int *s_i = reinterpret_cast<int *>(s_d + kRrtcWarps);
     int *s_misc = s_i + kRrtcWarps;                      // [8]
     unsigned char *act = reinterpret_cast<unsigned char *>(s_misc + 8);
-    ChunkScratch cs{};
-    if (CULL && CHUNK > 0) carve_chunk(p + rrtc_misc_bytes(), R, CHUNK, threadIdx.x / kWarp, cs);
     for (int j = threadIdx.x; j < R.L; j += blockDim.x) act[j] = R.active[j];
     __syncthreads();
 
@@ -437,8 +442,7 @@ __global__ void __launch_bounds__(kRrtcThreads, 5) k_rrtc(DevRobot R, DevEnv E, 
 
 // Batched planning: block b serves problem b % n as lane b / n, so every problem gets
 // lanes from the first wave of resident blocks.  The problem's descriptors are copied
-// into shared memory once.  Bounded to 128 registers (four blocks per SM): the chunked
-// edge checks otherwise take the kernel to 168.
+// into shared memory once.  Bounded to 128 registers: four blocks per SM.
 template <int SPL, bool CULL>
 __global__ void __launch_bounds__(kRrtcThreads, 4) k_rrtc_batch(const BatchProblem *__restrict__ probs, int n,
                                                             int lanes_per_problem, RrtcParams prm, int *rr) {
@@ -491,23 +495,33 @@ __global__ void __launch_bounds__(kRrtcThreads, 4) k_rrtc_batch(const BatchProbl
 }
 
 
+// Raises a kernel's dynamic shared-memory limit to `smem`; never lowers it.
+template <typename K>
+inline cudaError_t rrtc_raise_smem(K kern, size_t smem) {
+    cudaFuncAttributes fa;
+    const cudaError_t ce = cudaFuncGetAttributes(&fa, kern);
+    if (ce != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return ce;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 // Launcher of the single-problem kernel for spheres-per-lane counts A..A+3 (see
 // gbmp_rrtc.cuh).
 template <int SPL>
 inline cudaError_t rrtc_launch_one(bool cull, int grid, size_t smem, cudaStream_t st, const DevRobot &R,
                                    const DevEnv &E, const RrtcDev &P, const RrtcParams &prm) {
     auto kern = cull ? k_rrtc<SPL, true> : k_rrtc<SPL, false>;
-    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t ce = rrtc_raise_smem(kern, smem);
     if (ce != cudaSuccess) return ce;
     kern<<<grid, kRrtcThreads, smem, st>>>(R, E, P, prm);
     return cudaGetLastError();
 }
 
-template <int SPL>
-inline cudaError_t rrtc_batch_launch_one(bool cull, int grid, size_t smem, cudaStream_t st, const BatchProblem *probs,
-                                         int n, int lpp, const RrtcParams &prm, int *rr) {
-    auto kern = cull ? k_rrtc_batch<SPL, true> : k_rrtc_batch<SPL, false>;
-    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// (By chunks, CULL true, spheres per lane do not matter: SPL is 1.)
+template <int SPL, bool CULL>
+inline cudaError_t rrtc_batch_launch_one(int grid, size_t smem, size_t reserve, cudaStream_t st,
+                                         const BatchProblem *probs, int n, int lpp, const RrtcParams &prm, int *rr) {
+    auto kern = k_rrtc_batch<SPL, CULL>;
+    const cudaError_t ce = rrtc_raise_smem(kern, reserve);
     if (ce != cudaSuccess) return ce;
     kern<<<grid, kRrtcThreads, smem, st>>>(probs, n, lpp, prm, rr);
     return cudaGetLastError();
@@ -525,13 +539,13 @@ inline cudaError_t rrtc_batch_launch_one(bool cull, int grid, size_t smem, cudaS
     }
 
 #define GBMP_RRTC_DEFINE_BATCH_LAUNCHER(NAME, A)                                                              \
-    cudaError_t NAME(int spl, bool cull, int grid, size_t smem, cudaStream_t st, const BatchProblem *probs,   \
-                     int n, int lpp, const RrtcParams &prm, int *rr) {                                        \
+    cudaError_t NAME(int spl, int grid, size_t smem, size_t reserve, cudaStream_t st,                         \
+                     const BatchProblem *probs, int n, int lpp, const RrtcParams &prm, int *rr) {             \
         switch (spl) {                                                                                        \
-        case A: return rrtc_batch_launch_one<A>(cull, grid, smem, st, probs, n, lpp, prm, rr);                \
-        case A + 1: return rrtc_batch_launch_one<A + 1>(cull, grid, smem, st, probs, n, lpp, prm, rr);        \
-        case A + 2: return rrtc_batch_launch_one<A + 2>(cull, grid, smem, st, probs, n, lpp, prm, rr);        \
-        default: return rrtc_batch_launch_one<A + 3>(cull, grid, smem, st, probs, n, lpp, prm, rr);           \
+        case A: return rrtc_batch_launch_one<A, false>(grid, smem, reserve, st, probs, n, lpp, prm, rr);      \
+        case A + 1: return rrtc_batch_launch_one<A + 1, false>(grid, smem, reserve, st, probs, n, lpp, prm, rr);\
+        case A + 2: return rrtc_batch_launch_one<A + 2, false>(grid, smem, reserve, st, probs, n, lpp, prm, rr);\
+        default: return rrtc_batch_launch_one<A + 3, false>(grid, smem, reserve, st, probs, n, lpp, prm, rr); \
         }                                                                                                     \
     }
 

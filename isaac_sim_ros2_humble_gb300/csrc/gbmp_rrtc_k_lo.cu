@@ -7,15 +7,17 @@ namespace gbmp {
 GBMP_RRTC_DEFINE_LAUNCHER(rrtc_launch_lo, 1)
 
 // One problem with the edge checks by chunks, for every robot whose spheres a lane are then no
-// matter.  At most 168 registers: three blocks an SM measured 646 us at 1,024 lanes (the
-// shelf, range 0.1; as few as one block 654), four 736, five 842; k_rrtc 866.
+// matter.  Bounded to 168 registers it takes 120, so that four blocks fit on an SM.  At 1,024
+// lanes, p50 on the shelf (range 0.1) and ten problems without a path: 0.45 ms and 53 ms;
+// bounded to four blocks (111 registers) 0.46 and 54, to five with chunks of 4 (90
+// registers) 0.51 and 43; k_rrtc 0.68 and 67.
 __global__ void __launch_bounds__(kRrtcThreads, 3) k_rrtc_chunk(DevRobot R, DevEnv E, RrtcDev P, RrtcParams prm) {
     rrtc_lane<1, true, kRrtcSoloChunk>(R, E, P, prm, blockIdx.x);
 }
 
 cudaError_t rrtc_launch_chunk(int grid, size_t smem, cudaStream_t st, const DevRobot &R, const DevEnv &E,
                             const RrtcDev &P, const RrtcParams &prm) {
-    cudaError_t ce = cudaFuncSetAttribute(k_rrtc_chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t ce = rrtc_raise_smem(k_rrtc_chunk, smem);
     if (ce != cudaSuccess) return ce;
     k_rrtc_chunk<<<grid, kRrtcThreads, smem, st>>>(R, E, P, prm);
     return cudaGetLastError();
