@@ -21,6 +21,7 @@
 // lane iteration cap, the node cap and a %globaltimer deadline end the launch with a
 // status the host reads.
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -454,9 +455,10 @@ struct gbmp_batch_planner_s {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     unsigned long long *d_deadline = nullptr;   // [0] deadline, [1] round-robin counter
     std::vector<int> prev;                // 2 per problem
-    // captured graphs by launch shape (a few shapes, least recently used evicted)
+    // captured graphs by launch (a few, least recently used evicted)
+    using GraphKey = std::array<uint64_t, 16>;
     struct Captured {
-        long long key[12];
+        GraphKey key;
         cudaGraphExec_t exec;
         long long used;
     };
@@ -770,18 +772,21 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
     b->cur_n = n;
     GBMP_CUDA(cudaEventRecord(b->ev0, st));
     if (use_graph) {
-        float dd_f[3] = {prm.dd_alpha, prm.dd_radius, prm.dd_min};
-        unsigned dd_bits[3];
-        memcpy(dd_bits, dd_f, sizeof dd_bits);
-        unsigned tr_bits = 0;
-        memcpy(&tr_bits, &prm.tree_ratio, sizeof tr_bits);
-        const long long key[12] = {n, lanes_per_problem, (long long)smem, spl, cull, s->max_iters,
-                                   (long long)(lim * 1e6), (long long)(prm.range * 1e6) ^ ((long long)(prm.res * 1e9) << 20),
-                                   prm.dd ? (long long)dd_bits[0] | ((long long)dd_bits[1] << 32) : -1,
-                                   prm.dd ? (long long)dd_bits[2] : -1, prm.balance, (long long)tr_bits};
+        // everything a captured launch holds: its shape, the planning parameters and the time
+        // limit, to the bit
+        auto bits = [](float v) {
+            uint32_t u = 0;
+            memcpy(&u, &v, sizeof u);
+            return (uint64_t)u;
+        };
+        const gbmp_batch_planner_s::GraphKey key{
+            (uint64_t)n, (uint64_t)lanes_per_problem, (uint64_t)smem, (uint64_t)spl, (uint64_t)cull,
+            (uint64_t)prm.max_iters, (uint64_t)prm.rule, bits(prm.range), bits(prm.res), (uint64_t)(lim * 1e9),
+            (uint64_t)prm.dd, bits(prm.dd_alpha), bits(prm.dd_radius), bits(prm.dd_min), (uint64_t)prm.balance,
+            bits(prm.tree_ratio)};
         cudaGraphExec_t exec = nullptr;
         for (auto &g : b->graphs)
-            if (memcmp(key, g.key, sizeof key) == 0) { exec = g.exec; g.used = ++b->use_clock; }
+            if (key == g.key) { exec = g.exec; g.used = ++b->use_clock; }
         if (!exec) {
             if (b->graphs.size() >= 8) {
                 auto lru = std::min_element(b->graphs.begin(), b->graphs.end(),
@@ -803,7 +808,7 @@ gbmp_status batch_begin(gbmp_batch_planner b, int n, const gbmp_rrtc_problem *pr
             cudaGraphDestroy(g);
             if (ce != cudaSuccess) { set_error("graph instantiate failed: %s", cudaGetErrorString(ce)); return GBMP_ERR_CUDA; }
             gbmp_batch_planner_s::Captured c;
-            memcpy(c.key, key, sizeof key);
+            c.key = key;
             c.exec = exec;
             c.used = ++b->use_clock;
             b->graphs.push_back(c);
