@@ -152,8 +152,10 @@ bool scene_field_plan(const std::vector<double> &b, DevEnv &E, bool *tight) {
 
 cudaError_t scene_field_build(const DevEnv &E, float slack, float4 *field, cudaStream_t s) {
     const int cells = E.nx * E.ny * E.nz;
-    k_scene_field<<<(cells * kFieldLanes + 255) / 256, 256, 0, s>>>(E, slack, field);
-    return cudaGetLastError();
+    // the launch's own result: cudaGetLastError would also report what an earlier call left
+    DevEnv e = E;
+    void *args[] = {&e, &slack, &field};
+    return cudaLaunchKernel((const void *)k_scene_field, dim3((cells * kFieldLanes + 255) / 256), dim3(256), args, 0, s);
 }
 
 }  // namespace gbmp
