@@ -76,6 +76,12 @@ __global__ void __launch_bounds__(256) k_scene_field(DevEnv E, float slack, floa
         n.add(d2, o2);
         n.add(d3, 0xffff);   // below d1 and d2, so it ends as a third distance at most
     }
+    // A cell that no distance could be computed for names obstacle 0 and says nothing: a state
+    // that is no number is tested against what its cell names.
+    if (n.o1 == 0xffff) {
+        n.d1 = n.d2 = n.d3 = -3.0e38f;
+        n.o1 = 0;
+    }
     if (in && o0 == 0) field[cell] = make_float4(n.d1, n.d2, n.d3, __int_as_float(n.o1 | n.o2 << 16));
 }
 

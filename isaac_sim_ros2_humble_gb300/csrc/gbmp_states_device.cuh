@@ -86,7 +86,7 @@ __device__ __forceinline__ bool sphere_open(const SmemTables &t, const DevEnv &E
     float way;
     const float4 f = __ldg(scene_cell(E, c.x, c.y, c.z, way));
     if (f.x - way > rad) return false;
-    const unsigned ids = __float_as_uint(f.w);
+    const unsigned ids = __float_as_uint(f.w);   // the first always names an obstacle (k_scene_field)
     h = obstacle_hit(t, E, (int)(ids & 0xffffu), c, r);
     if (!h && !(f.y - way > rad)) {
         if ((ids >> 16) != 0xffffu) h = obstacle_hit(t, E, (int)(ids >> 16), c, r);

@@ -94,3 +94,25 @@ def test_verdicts_and_work(which):
     links = len(np.unique(robot.sphere_link))
     all_obstacles = links * (9 * ns + 33 * nb + 34 * nc)     # flops of one test of each kind
     assert work(E) <= work(api.Env(W.Environment.empty())) + 2 * all_obstacles
+
+
+@pytest.mark.parametrize("obstacle", ["sphere", "cylinder"])
+@pytest.mark.parametrize("far", [0.0, 9e17])
+def test_states_that_are_no_numbers_near_one_obstacle(obstacle, far):
+    """A cell of a field with one obstacle names one; a state that is no number meets it, and
+    collides just where it is a cylinder, whose clamps drop the NaN."""
+    robot = W.serial_arm(79, dof=7, n_spheres=40)
+    e = W.Environment.empty()
+    if obstacle == "sphere":
+        e.sphere_pos, e.sphere_r = f([[0.4 + far, 0.2, 0.5]]), f([0.1])
+    else:
+        e.cyl_pos, e.cyl_rot = f([[0.4 + far, 0.2, 0.5]]), np.eye(3, dtype=f)[None]
+        e.cyl_radius, e.cyl_height = f([0.1]), f([0.4])
+    R, E = api.Robot(robot), api.Env(e)
+    q = torch.from_numpy(robot.sample_full(np.random.default_rng(2), 65)).cuda()
+    q[::2, 1] = float("nan")
+    v, total = torch.full((65,), 9, dtype=torch.uint8, device="cuda"), torch.zeros(65, device="cuda")
+    api.check_states(R, E, q, v, None, total, _lib.CHECK_COST)
+    torch.cuda.synchronize()
+    assert (v[::2] == (obstacle == "cylinder")).all()
+    np.testing.assert_array_equal(_check(R, E, q)[::2], v.cpu().numpy()[::2])
