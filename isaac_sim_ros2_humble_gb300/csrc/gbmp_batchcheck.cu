@@ -10,6 +10,9 @@
 // bit-identical to a gbmp_check_states_fk call of its own.  Shared memory is sized for the
 // largest request; the spheres-per-lane template of the costs covers the robot with the
 // most spheres (smaller robots leave slots empty).
+#include <algorithm>
+#include <new>
+
 #include "gbmp_states_device.cuh"
 
 namespace gbmp {
@@ -129,6 +132,13 @@ gbmp_status gbmp_check_batch_create(int32_t max_requests, gbmp_check_batch *out)
         if (cudaMallocHost(&b->h_buf, b->bytes) != cudaSuccess || cudaMalloc(&b->d_buf, b->bytes) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming) != cudaSuccess) {
             set_error("check batch: allocation of %zu bytes failed", b->bytes);
+            st = GBMP_ERR_OUT_OF_MEMORY;
+            break;
+        }
+        try {   // so that a call allocates nothing
+            b->order.reserve((size_t)max_requests);
+        } catch (const std::bad_alloc &) {
+            set_error("check batch: out of host memory for %d requests", max_requests);
             st = GBMP_ERR_OUT_OF_MEMORY;
         }
     } while (false);
