@@ -853,6 +853,7 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     DevEnv &E = e->view;
     E.ns = ns; E.nb = nb; E.nc = nc;
     std::vector<double> bounds;
+    bounds.reserve(4 * ((size_t)ns + nb + nc));
     auto bound = [&](const std::vector<double> &c, const std::vector<double> &r) {
         for (size_t i = 0; i < r.size(); ++i) bounds.insert(bounds.end(), {c[3 * i], c[3 * i + 1], c[3 * i + 2], r[i]});
     };
@@ -870,14 +871,14 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     }
     const size_t ubytes = sizeof(float4) * upload.size();
     cudaError_t err = cudaMalloc(&e->d_words, ubytes + (field ? sizeof(float4) * (size_t)E.nx * E.ny * E.nz : 0));
-    if (err == cudaSuccess) err = cudaMemcpy(e->d_words, upload.data(), ubytes, cudaMemcpyHostToDevice);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(e->d_words, upload.data(), ubytes, cudaMemcpyHostToDevice, nullptr);
     E.words = e->d_words;
     if (err == cudaSuccess && field) {
         float4 *values = e->d_words + e->h_words.size();
         err = scene_field_build(E, kFieldSlack + (float)(6.0 * skew), values, nullptr);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
         E.field = values;
     }
+    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
     if (err != cudaSuccess) {
         set_error("uploading environment failed: %s", cudaGetErrorString(err));
         gbmp_env_destroy(e);

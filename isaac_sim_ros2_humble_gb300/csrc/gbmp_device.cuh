@@ -119,7 +119,7 @@ struct DevEnv {
 
 // Cells along the field's longest side (512 KB a scene at most).  65,536 edges of the 8-DOF
 // arm in 336 obstacles: 1.255 ms with 32, 1.242 with 48, 1.238 with 64, 1.233 with 128;
-// a scene of 336 obstacles takes 45 us longer to create (76 us; some 60 us longer with 48).
+// a scene of 336 obstacles takes some 40 us longer to create (68 us).
 constexpr int kFieldCells = 32;
 constexpr double kFieldBorder = 0.2;     // metres of field around the obstacles
 constexpr double kFieldLargest = 1.0;    // bounding radius of the obstacles that span the field
