@@ -22,6 +22,7 @@ void set_error(const char *fmt, ...) {
     vsnprintf(buf, sizeof buf, fmt, ap);
     va_end(ap);
     g_err = buf;
+    cudaGetLastError();   // reported: the next launch of this thread starts without it
 }
 
 // ---------------------------------------------------------------------------------
