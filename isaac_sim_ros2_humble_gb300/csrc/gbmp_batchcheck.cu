@@ -210,7 +210,7 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
         CheckTask &T = tasks[nt++];
         T.R = cost ? q.robot->dev : q.robot->dev_chunk;
         T.R.work = work;
-        T.E = q.env->dev_states();
+        T.E = q.env->dev();
         T.q = q.d_q;
         T.n = q.n;
         T.verdict = q.d_verdict;

@@ -779,8 +779,9 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     }
     // Bounding spheres hold for rotations: with rows off orthonormal by e an obstacle reaches
     // 6 e of its size farther at most.  Up to half of kBroadMargin, which the tests that use
-    // the spheres add, is let pass; more, or a number that is not finite, makes the scene loose.
-    // So does an obstacle so far away that the squares of a run's sphere overflow.
+    // the spheres add, is let pass; more, or a number that is not finite, makes the scene
+    // loose: it has no field, and no test passes over a run of obstacles.  So does an obstacle
+    // so far away that the squares of a run's sphere overflow.
     double skew = 0.0;
     bool loose = false;
     const double overflow = 1e18;
@@ -851,6 +852,9 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     cluster_spheres(sc, srd, os, runs);
     cluster_spheres(bc, brd, ob, runs + env_clusters(ns));
     cluster_spheres(cc, crd, oc, runs + env_clusters(ns) + env_clusters(nb));
+    if (loose)   // every run reaches everywhere
+        for (float4 *run = runs; run != e->h_words.data() + words; ++run)
+            *run = make_float4(0.f, 0.f, 0.f, std::numeric_limits<float>::infinity());
     DevEnv &E = e->view;
     E.ns = ns; E.nb = nb; E.nc = nc;
     std::vector<double> bounds;
@@ -861,18 +865,12 @@ gbmp_status gbmp_env_create(int32_t ns, const float *sp, const float *sr, int32_
     bound(sc, srd);
     bound(bc, brd);
     bound(cc, crd);
-    e->loose = loose;
     e->tight = bounds.empty();
     const bool field = !loose && scene_field_plan(bounds, E, &e->tight);
-    std::vector<float4> upload(e->h_words);
-    if (loose) {
-        upload.insert(upload.end(), e->h_words.begin(), e->h_words.end());
-        for (size_t i = upload.size() - env_clusters(ns) - env_clusters(nb) - env_clusters(nc); i < upload.size(); ++i)
-            upload[i] = make_float4(0.f, 0.f, 0.f, std::numeric_limits<float>::infinity());
-    }
-    const size_t ubytes = sizeof(float4) * upload.size();
-    cudaError_t err = cudaMalloc(&e->d_words, ubytes + (field ? sizeof(float4) * (size_t)E.nx * E.ny * E.nz : 0));
-    if (err == cudaSuccess) err = cudaMemcpyAsync(e->d_words, upload.data(), ubytes, cudaMemcpyHostToDevice, nullptr);
+    const size_t wbytes = sizeof(float4) * e->h_words.size();
+    cudaError_t err = cudaMalloc(&e->d_words, wbytes + (field ? sizeof(float4) * (size_t)E.nx * E.ny * E.nz : 0));
+    if (err == cudaSuccess)
+        err = cudaMemcpyAsync(e->d_words, e->h_words.data(), wbytes, cudaMemcpyHostToDevice, nullptr);
     E.words = e->d_words;
     if (err == cudaSuccess && field) {
         float4 *values = e->d_words + e->h_words.size();
@@ -922,7 +920,7 @@ gbmp_status gbmp_check_states_fk(gbmp_robot r, gbmp_env env, const float *d_q, i
     GBMP_CHECK_ARG(mode == GBMP_CHECK_VERDICT || mode == GBMP_CHECK_COST, "unknown mode %d", mode);
     if (n == 0) return GBMP_OK;
     GBMP_CHECK_ARG(d_q, "q is NULL");
-    const DevEnv E = env->dev_states();
+    const DevEnv E = env->dev();
     cudaStream_t s = (cudaStream_t)stream;
     const int nwords = env_words(E.ns, E.nb, E.nc);
     gbmp_status st = GBMP_OK;

@@ -206,8 +206,7 @@ cudaError_t scene_field_build(const DevEnv &E, float slack, float4 *field, cudaS
 
 struct gbmp_env_s {
     int ns = 0, nb = 0, nc = 0;
-    // One allocation: the words, then the field or, in a loose scene, the words of state checks.
-    float4 *d_words = nullptr;
+    float4 *d_words = nullptr;   // one allocation: the words, then the field
     std::vector<float4> h_words;
     gbmp::DevEnv view{};
     // The field says almost all there is to say (cells of at most kFieldFine, no obstacle
@@ -217,14 +216,5 @@ struct gbmp_env_s {
     // 2,260 obstacles with cells of 0.14 m, 70,000 states: 8-DOF arm 208 us one at a time, 166
     // together; 38-DOF arm 643 and 672.
     bool tight = false;
-    // An obstacle may reach beyond its bounding sphere (an unbounded box, a rotation that is
-    // none).  The scene has no field; the runs of obstacles that state checks read reach
-    // everywhere, and plans of one problem go state by state.
-    bool loose = false;
     gbmp::DevEnv dev() const { return view; }
-    gbmp::DevEnv dev_states() const {
-        gbmp::DevEnv e = view;
-        if (loose) e.words += h_words.size();
-        return e;
-    }
 };

@@ -708,7 +708,7 @@ extern "C" gbmp_status gbmp_constrained_motions(gbmp_robot r, gbmp_env env, cons
         p.reference[k] = proj->reference[k];
         p.tolerance[k] = proj->tolerance[k];
     }
-    const DevEnv E = env->dev_states();
+    const DevEnv E = env->dev();
     DevRobot D = r->dev_chunk;
     D.work = nullptr;
     const int nwords = env_words(E.ns, E.nb, E.nc);

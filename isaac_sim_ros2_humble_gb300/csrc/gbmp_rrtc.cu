@@ -339,9 +339,8 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     // next to the scene: faster at every lane count, with a path and without (p50 of 48
     // problems on the shelf, range 0.1: 1 lane 2.44 -> 1.83 ms, 64 lanes 0.51 -> 0.35, 456
     // lanes 0.55 -> 0.41, 1,024 lanes 0.68 -> 0.45; problems of the uneven mix without a path:
-    // 64 lanes 620 -> 415 ms, 1,024 lanes 68 -> 53 ms).  Chunks pass over runs of obstacles, so
-    // not in a loose scene
-    const bool chunk = r->dev_chunk.cull && !env->loose &&
+    // 64 lanes 620 -> 415 ms, 1,024 lanes 68 -> 53 ms).
+    const bool chunk = r->dev_chunk.cull &&
                        std::max(rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk), rrtc_block_smem(r->dev, nwords, 0)) <=
                            kSmemLimit;
     DevRobot DR = chunk ? r->dev_chunk : r->dev;

@@ -75,3 +75,35 @@ def test_plans_against_the_oracle(which):
             states = m.edge_states(path[i], path[i + 1], 0.02, _lib.STEP_LINF)
             assert np.abs(m.clearance(states[fh[i]: fh[i] + 1])).max() <= 1e-4
     assert solved >= 4
+
+
+def _with_sphere(env, p):
+    return dataclasses.replace(env, sphere_pos=np.concatenate([env.sphere_pos, np.float32([p])]),
+                               sphere_r=np.concatenate([env.sphere_r, np.float32([0.1])]))
+
+
+@pytest.mark.parametrize("form", [0, 1, 4])
+@pytest.mark.parametrize("which", ["half-space", "scaled boxes", "scaled cylinders", "nearly", "-infinity", "-1e20 m"])
+def test_edges_against_the_oracle(which, form):
+    robot = W.serial_arm(82, dof=7, n_spheres=70)
+    env = _scene(which)
+    if which[0] == "-":
+        env = _with_sphere(W.random_env(81, 90, 6, 3, oriented=True), (float(which.split()[0].replace("inity", "")), 0, 0))
+    R, E, m = api.Robot(robot), api.Env(env), O.OracleModel(robot, env)
+    n = 300
+    q = robot.sample_full(np.random.default_rng(11), 2 * n)
+    a, b = q[:n], (q[:n] + 0.3 * (q[n:] - q[:n])).astype(np.float32)
+    ok, okv = (torch.full((n,), 9, dtype=torch.uint8, device="cuda") for _ in range(2))
+    fh = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+    R.set_edge_form(form)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    api.check_edges(R, E, da, db, 0.05, _lib.STEP_LINF, ok, fh)
+    api.check_edges(R, E, da, db, 0.05, _lib.STEP_LINF, okv)
+    torch.cuda.synchronize()
+    assert torch.equal(ok, okv)
+    o_ok, o_fh, _, _ = m.check_motions(a, b, 0.05, _lib.STEP_LINF)
+    assert 0.1 < o_ok.mean() < 0.9
+    fh = fh.cpu().numpy()
+    for k in np.nonzero(fh != o_fh)[0]:     # a state at the surface decided otherwise
+        s = [x for x in (fh[k], o_fh[k]) if x >= 0]
+        assert np.abs(m.clearance(m.edge_states(a[k], b[k], 0.05, _lib.STEP_LINF)[min(s): min(s) + 1]))[0] <= 1e-4
