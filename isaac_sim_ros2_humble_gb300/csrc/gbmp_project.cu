@@ -356,6 +356,7 @@ __device__ __forceinline__ void proj_costs(const DevRobot &R, const ProjParams &
 
 // checkStates on the nb recorded states in w.rec: true when every one is collision-free and
 // has no task-space and no limit cost (proj_costs' arithmetic, one state a lane).
+template <bool TIGHT>
 __device__ __forceinline__ bool recorded_pass(const SmemTables &t, const DevRobot &R, const DevEnv &E,
                                               const ProjParams &p, const ProjScratch &w, int nb, int lane) {
     const int L = R.L;
@@ -391,7 +392,7 @@ __device__ __forceinline__ bool recorded_pass(const SmemTables &t, const DevRobo
         }
     }
     if (__any_sync(kFull, bad)) return false;
-    return warp_verdicts<false, false>(t, R, E, w.sc, nb, lane) == 0u;
+    return warp_verdicts<false, TIGHT>(t, R, E, w.sc, nb, lane) == 0u;
 }
 
 template <int U>
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
 // achieved (checkAchieveGoal).  ok = achieved and every recorded state passed; cost = L2
 // length over all joints of the recorded states; count = recorded states (the first
 // `cap` are written to `states` when it is not null).
-template <int U>
+template <int U, bool TIGHT>
 __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
     k_constrained_motion(DevRobot R, DevEnv E, ProjParams p, const float *__restrict__ from,
                          const float *__restrict__ to, long long n, float res, int max_iters,
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
                     if (lane + kWarp * u < L) w.rec[waiting * L + lane + kWarp * u] = q[u];
                 __syncwarp();
                 if (++waiting == kCheckStates) {
-                    feasible = recorded_pass(t, R, E, p, w, waiting, lane);
+                    feasible = recorded_pass<TIGHT>(t, R, E, p, w, waiting, lane);
                     waiting = 0;
                 }
             }
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp)
                 break;
             }
         }
-        if (achieved && feasible && waiting) feasible = recorded_pass(t, R, E, p, w, waiting, lane);
+        if (achieved && feasible && waiting) feasible = recorded_pass<TIGHT>(t, R, E, p, w, waiting, lane);
         if (lane == 0) {
             const bool ok = achieved && feasible;
             if (ok_out) ok_out[s] = ok;
@@ -712,7 +713,10 @@ extern "C" gbmp_status gbmp_constrained_motions(gbmp_robot r, gbmp_env env, cons
     DevRobot D = r->dev_chunk;
     D.work = nullptr;
     const int nwords = env_words(E.ns, E.nb, E.nc);
-    const void *fn = r->L <= kWarp ? (const void *)k_constrained_motion<1> : (const void *)k_constrained_motion<2>;
+    const void *fn = env->tight ? r->L <= kWarp ? (const void *)k_constrained_motion<1, true>
+                                                : (const void *)k_constrained_motion<2, true>
+                     : r->L <= kWarp ? (const void *)k_constrained_motion<1, false>
+                                     : (const void *)k_constrained_motion<2, false>;
     gbmp_status st = ensure_smem_optin(fn);
     if (st) return st;
     int warps = 0, per_sm = 0;
