@@ -338,8 +338,8 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     // by chunks of states where the tables allow it (at most 32 groups) and the scratch fits
     // next to the scene: faster at every lane count, with a path and without (p50 of 48
     // problems on the shelf, range 0.1: 1 lane 2.44 -> 1.83 ms, 64 lanes 0.51 -> 0.35, 456
-    // lanes 0.55 -> 0.41, 1,024 lanes 0.68 -> 0.45; problems of the uneven mix without a path:
-    // 64 lanes 620 -> 415 ms, 1,024 lanes 68 -> 53 ms).
+    // lanes 0.55 -> 0.41, 1,024 lanes 0.68 -> 0.42; problems of the uneven mix without a path:
+    // 64 lanes 620 -> 415 ms, 1,024 lanes 67 -> 57 ms)
     const bool chunk = r->dev_chunk.cull &&
                        std::max(rrtc_block_smem(r->dev_chunk, nwords, kRrtcSoloChunk), rrtc_block_smem(r->dev, nwords, 0)) <=
                            kSmemLimit;
@@ -359,6 +359,7 @@ gbmp_status gbmp_rrtc_solve_goals(gbmp_planner p, gbmp_env env, const float *h_s
     prm.dd_min = s->dd_min_radius;
     prm.balance = balance;
     prm.tree_ratio = tree_ratio;
+    if (s->max_iters >= 64 * kRrtcEarlyIters) prm.early = kRrtcEarlyBlocks * r->num_sms;
     // device deadline: set by the reset kernel
     prm.deadline_ns = 0;
     prm.deadline_ptr = (unsigned long long *)(D.state + 8);

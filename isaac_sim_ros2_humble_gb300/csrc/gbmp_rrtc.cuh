@@ -17,12 +17,19 @@ constexpr int kRrtcThreads = kRrtcWarps * kWarp;
 // shelf at range 0.5, 25 states an edge: 546 us a problem with 4, 530 with 8, 528 with 10.
 constexpr int kRrtcChunk = 4;
 constexpr int kRrtcSoloChunk = 8;
+// Single-problem plans by chunks: lanes beyond kRrtcEarlyBlocks an SM join once a lane has done
+// kRrtcEarlyIters iterations (or after kRrtcEarlyPolls microseconds).  Four blocks fit on an SM,
+// which a problem without a path needs (its lanes read whole trees); a problem that is solved
+// within some tens of iterations only waits longer for each.  1,024 lanes, p50 on the shelf and ten
+// problems without a path: all lanes at once 0.45 ms and 53 ms; three blocks 0.42 and 71; this
+// 0.42 and 57 (64 iterations 0.42 and 59, 128: 0.43 and 61).  Only where a lane may do 64 times
+// as many iterations.
+constexpr int kRrtcEarlyBlocks = 3, kRrtcEarlyIters = 32, kRrtcEarlyPolls = 2000;
 
 // Shared memory of a planning block: staged tables, the lane's joint vectors and flags, and
 // four scratches: of chunks of `chunk` states where the edge checks run by chunks (robots of at
-// most 32 sphere groups), else of a state.  (While the chunk forms held both, three blocks
-// of the single-problem kernel fitted on an SM instead of four, and ten problems without a path took 71 ms
-// at 1,024 lanes; 53 ms now, 67 with k_rrtc.)
+// most 32 sphere groups), else of a state.  (While the chunk forms held both, three blocks of
+// the single-problem kernel fitted on an SM instead of four.)
 __host__ __device__ inline size_t rrtc_misc_bytes() { return align16(6 * kMaxLinks * 4 + 256); }
 __host__ __device__ inline size_t rrtc_block_smem(const DevRobot &R, int nwords, int chunk) {
     return smem_tables_bytes(R, nwords) + rrtc_misc_bytes() +
@@ -53,6 +60,7 @@ struct RrtcParams {
     const unsigned long long *deadline_ptr;   // read from device memory when non-null
     int dd = 0;                       // dynamic domain on (needs RrtcDev::radii)
     float dd_alpha = 0.f, dd_radius = 0.f, dd_min = 0.f;
+    int early = 0x7fffffff;           // lanes from this one on join late (k_rrtc_chunk)
     int balance = 3;                  // 0 none, 1 pRRTC size, 2 pRRTC swap, 3 proportional
     float tree_ratio = 0.5f;
 };

@@ -55,3 +55,34 @@ def test_forms(dof, n_spheres, obstacles, chunks, lanes):
             states = om.edge_states(path[i], path[i + 1], 0.03, _lib.STEP_LINF)
             assert np.abs(om.clearance(states[fh[i]: fh[i] + 1])).max() <= 1e-4
     assert solved
+
+
+@pytest.mark.parametrize("lanes", [457, 700])
+@pytest.mark.parametrize("max_iters", [60, 2048, 100000])
+def test_lanes_that_join_late(lanes, max_iters):
+    """More lanes than start at once: a path as soon as there is one, all lanes' iterations where
+    there is none, and an end at the deadline."""
+    m = W.serial_arm(1, dof=7, n_spheres=59)
+    env = W.shelf_env(4)
+    R, E, om = api.Robot(m), api.Env(env), O.OracleModel(m, env)
+    q = m.sample_full(np.random.default_rng(5), 200)
+    free = q[om.clearance(q) > 1e-3]
+    planner = api.Planner(R, max_nodes=60000, path_cap=2048)
+    kw = dict(lanes=lanes, max_iters=max_iters, range_=0.3, resolution=0.02, rule=_lib.STEP_LINF)
+    for k in range(6):
+        res, path = planner.solve(E, free[2 * k], free[2 * k + 1], seed=k, **kw)
+        assert res["solved"]
+        ok, fh, _, _ = om.check_motions(path[:-1], path[1:], 0.02, _lib.STEP_LINF)
+        for i in np.nonzero(~ok)[0]:
+            states = om.edge_states(path[i], path[i + 1], 0.02, _lib.STEP_LINF)
+            assert np.abs(om.clearance(states[fh[i]: fh[i] + 1])).max() <= 1e-4
+    # hardly a way out where a shell of obstacles surrounds the tip: a cap or the deadline may end it
+    c = W.sphere_centers_numpy(m, free[:1])[0]
+    pts = c[-1] + 0.25 * np.asarray([W._unit(np.random.default_rng(k)) for k in range(400)])
+    pts = pts[(np.linalg.norm(pts[:, None] - c, axis=-1) - m.sphere_r > 0.045).all(1)].astype(np.float32)
+    shell = W.Environment.empty()
+    shell.sphere_pos, shell.sphere_r = pts, np.full(len(pts), 0.04, np.float32)
+    res, _ = planner.solve(api.Env(shell), free[0], free[1], seed=1, time_limit_s=0.5, **kw)
+    assert res["solved"] or res["status"] in (2, 3, 4)
+    if res["status"] == 3:
+        assert res["iterations"] == max_iters
