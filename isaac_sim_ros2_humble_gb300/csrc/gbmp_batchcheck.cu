@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
 }
 
 // `ks` states a warp at a time.  256 requests over 4 robots and 16 scenes, 1.57 million
-// states: 5.38 ms with one warp for each state, 1.53 ms now.
+// states: 5.38 ms with one warp for each state, 1.46 ms now.
 template <bool CNT, bool TIGHT>
 __global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStatesWarps)
     k_batch_verdicts(const CheckTask *__restrict__ tasks, const CheckRange *__restrict__ ranges, int ks) {
@@ -259,8 +259,8 @@ gbmp_status gbmp_check_batch_run(gbmp_check_batch b, const gbmp_check_request *r
             return GBMP_ERR_CAPACITY;
         }
     }
-    // states per block: about eight waves over all requests (1.53 ms on the 256-request mix
-    // above; four: 1.57, sixteen: 1.52), at least one round of its warps
+    // states per block: about eight waves over all requests (when it was chosen, 1.53 ms on
+    // the 256-request mix above; four: 1.57, sixteen: 1.52), at least one round of its warps
     const long long unit = (long long)sh.warps * sh.ks;
     const long long target = (long long)std::min(8 * sh.per_sm, kBatchBlocksPerSm) * b->num_sms;
     long long spb = (total + target - 1) / target;

@@ -1,6 +1,6 @@
-// gbmp_chunk.cu -- the edge-validation kernel (one warp per edge, the edge's states in
-// chunks of consecutive states; the chunk routines are in gbmp_chunk_device.cuh), its
-// launch set-up, and FK alone by chunks of consecutive states (gbmp_fk).
+// gbmp_chunk.cu -- the edge-validation kernel (edges cut into parts that warps take, their
+// states in chunks of consecutive states; the chunk routines are in gbmp_chunk_device.cuh),
+// its launch set-up, and FK alone by chunks of consecutive states (gbmp_fk).
 #include "gbmp_order.h"
 #include "gbmp_states_device.cuh"
 
@@ -8,8 +8,9 @@ namespace gbmp {
 
 // Warps per block of the chunk kernel: three blocks of 8 warps per SM at 80 registers.
 // The kernel is bound by instruction issue (0.72 of the issue slots at 65,536 edges), so
-// more warps bring little: 2.46 ms with two blocks, 2.22 ms with three, 2.21 ms with two
-// blocks of 16 warps at 64 registers (65,536 edges of the 8-DOF arm, verdicts).
+// more warps bring little: before scenes had a distance field, 2.46 ms with two blocks, 2.22
+// with three, 2.21 with two blocks of 16 warps at 64 registers (65,536 edges of the 8-DOF
+// arm, verdicts; 1.21 ms a call now).
 constexpr int kChunkWarps = 8;
 
 // Edge validation by chunks.  An edge's chunks, in their order, are cut into parts of
@@ -25,7 +26,8 @@ constexpr int kChunkWarps = 8;
 // Why parts: the free edges are few (18 % of the benchmark's) and long, so with one warp
 // per edge most warps idled while some walked up to 56 chunks in a row: 64 edges 0.47 ms
 // whole, 0.046 ms in parts; 3,001 edges of a 30-link robot with first hits 1.20 and 0.30
-// ms; 65,536 edges (18 for each warp) 2.22 and 2.26 ms (these with the kernel of that time).
+// ms; 65,536 edges (18 for each warp) 2.22 and 2.26 ms (all with the kernel of that time; now
+// 0.035, 0.26 and 1.21 ms).
 //
 // The chunk orders are gbmp_order.h's: state order when the first hit is asked for,
 // coarse to fine when only the verdict is.  On the 65,536 edges of the 8-DOF benchmark
@@ -34,15 +36,15 @@ constexpr int kChunkWarps = 8;
 // order), 4 passes 5.06 M, a full bit-reversed order of the chunks 4.96 M.
 //
 // The chunk's states are tested side by side in the lanes (gbmp_chunk_device.cuh).
-// 65,536 edges, verdicts: 2.22 ms; 3.79 ms when the states were walked one by one, their
-// spheres in the lanes.
+// When that came, 65,536 edges went from 3.79 ms (the states walked one by one, their spheres
+// in the lanes) to 2.22 ms.
 
 // A warp that holds a later part of an edge waits, at most kProbePolls looks, until the
-// edge's probes are known or it has a hit (bits beside the state count).  The warp that holds them took
-// them before this one took its item and does not wait before it has walked them.  Without
-// the wait a batch whose edges collide at once had every part of every edge walked: 161
-// edges 180 us, 54 us with it (63 us with one warp an edge); 64 edges take 40 us
-// with it, 35 without.
+// edge's probes are known or it has a hit (bits beside the state count).  The warp that holds
+// them took them before this one took its item and does not wait before it has walked them.
+// Without the wait a batch whose edges collide at once had every part of every edge walked: 161
+// edges 180 us, 54 us with it (63 us with one warp an edge); 64 edges took 40 us with it, 35
+// without.
 constexpr int kProbed0 = 1 << 28, kProbed1 = 1 << 29, kHit = 1 << 30, kStepsMask = kProbed0 - 1;
 constexpr int kProbePolls = 4096;
 constexpr int kMaxGrab = 8;   // settled items taken at a time in a batch of few edges

@@ -32,7 +32,7 @@
 // edges 0.3 obstacle candidates and 2.3 group pairs, each pair's test a chain of
 // shared-memory loads over 7 spheres.  Side by side the chunk's 23 (state, pair) items fill
 // a warp (3.8 -> 2.2 ms).  And the size of the code counts: the chunk kernel's loops are not unrolled
-// (51 KB instead of 75 KB; 65,536 edges 1.21 against 1.25 ms), for the instruction cache
+// (51 KB instead of 75 KB; 65,536 edges 1.21 against 1.25 ms a call), for the instruction cache
 // holds about one such body.
 #pragma once
 

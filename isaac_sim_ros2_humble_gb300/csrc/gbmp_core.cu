@@ -108,9 +108,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock *kWarp, 4)
 }
 
 // Collision verdicts of n states, `ks` states a warp at a time (gbmp_states_device.cuh).
-// One warp for each state, testing every obstacle against every group sphere, took 14.4 us
-// for the 4,096 configurations of the plain workload with their poses (12.3 us now), 250 us
-// for 70,072 states of a 9-DOF arm in 223 obstacles (75 us).
+// One warp for each state, testing every obstacle against every group sphere, took 250 us for
+// 70,072 states of a 9-DOF arm in 223 obstacles (75 us).  The 4,096 configurations of the plain
+// workload with their poses are one pass of half the resident warps either way: 8.6 us on the
+// device now, of it the staging of the tables and a chain of waits (0.39 of the issue slots).
 template <bool CNT, bool TIGHT>
 __global__ void __launch_bounds__(kStatesWarps *kWarp, kStatesResident / kStatesWarps)
     k_check_verdicts(DevRobot R, DevEnv E, const float *__restrict__ q, long long n, int ks,
@@ -174,9 +175,9 @@ __global__ void k_edge_setup(const float *__restrict__ from, const float *__rest
 // that cuts the edges into items: parts of `span` chunks so that a quarter of all chunks
 // (what is left of them when the colliding edges stop early) gives each warp about
 // kItemsPerWarp items, up to kEdgeMaxParts parts for the longest edge, and `grab` items a time
-// so that each warp comes back about kGrabsPerWarp times (65,536 edges: 2.26 ms with 32,
-// 2.32 with 16, 2.45 with 8; 17,339 shorter edges 0.312, 0.318 and 0.373 ms; 4 or 16 items
-// a warp instead of 8 cost up to 10 % on batches of 17,000 to 33,000 edges).
+// so that each warp comes back about kGrabsPerWarp times (with the kernel of that time, 65,536
+// edges: 2.26 ms with 32, 2.32 with 16, 2.45 with 8; 17,339 shorter edges 0.312, 0.318 and 0.373
+// ms; 4 or 16 items a warp instead of 8 cost up to 10 % on batches of 17,000 to 33,000 edges).
 constexpr int kItemsPerWarp = 8, kGrabsPerWarp = 32, kMaxSpan = 8;
 // First place of every bucket in the order, from the buckets' counts; and, where `plan` is
 // given, the plan of parts.  One warp.
@@ -426,9 +427,9 @@ static gbmp_status pack_tables(gbmp_robot_s *r, int piece, void **block, DevRobo
     r->h_jl = jl;
     r->h_axn = axn;
     r->h_axr = axr;
-    // Sphere groups (gbmp_groups.h) and their bounding spheres.  Pieces of links stay
-    // within min(kMaxGroups, 3 L) groups: the chunk kernels keep K x G group centres where
-    // the chunk's K x L pose rows were.
+    // Sphere groups (gbmp_groups.h) and their bounding spheres.  Pieces of links stay within
+    // min(kMaxGroups, 3 L) groups (3 L is the room that a former scratch layout had for their
+    // centres; more was not measured).
     std::vector<int> glink, sgrp;
     split_sphere_groups(L, S, r->slink.data(), r->sph_pos.data(), piece, piece > 0 ? std::min(kMaxGroups, 3 * L) : 0,
                         glink, sgrp);
@@ -1016,7 +1017,8 @@ gbmp_status gbmp_robot_set_edge_form(gbmp_robot r, int32_t form) {
 // Both entry points run the same kernels; they differ only in where the working memory
 // comes from: gbmp_check_edges grows a buffer owned by the robot handle, and
 // gbmp_check_edges_noalloc uses one fixed array that the library holds on each device.
-// Three launches, no host round trip:
+// Three launches, no host round trip (k_edge_few does the first two and their memset's work for
+// up to kFewEdges edges, unless a robot's generated set-up does the first):
 //   k_edge_setup   step count, direction and length per edge, length histogram;
 //   k_edge_order   the edges in longest-first order (counting sort by buckets), the
 //                  outputs of edges without a collision, and the plan of parts;
@@ -1026,8 +1028,9 @@ gbmp_status gbmp_robot_set_edge_form(gbmp_robot r, int32_t form) {
 // Working memory of E edges of L links:
 //   nsteps[E], order[E]   int
 //   dir[E*L]              float
-//   ctr[kEdgeCtrInts]     int    MUST START AT ZERO (hist[64], cursor[64], next; then
-//                                the EdgePlan): zeroed on the stream by every call
+//   ctr[kEdgeCtrInts]     int    hist[64], cursor[64], next, then the EdgePlan: zeroed on the
+//                                stream by every call that launches k_edge_setup or its
+//                                generated form; k_edge_few sets next and the plan itself
 // ---------------------------------------------------------------------------------
 namespace gbmp {
 
@@ -1144,7 +1147,7 @@ static gbmp_status edge_validate(gbmp_robot r, gbmp_env env, const float *d_from
 //   [0, 4 Ei)            nsteps[E]
 //   [4 Ei, 8 Ei)         order[E]
 //   [8 Ei, +4 D)         dir[E*L]
-//   [.., +4 C)           ctr[C]     zeroed on the stream at the start of every call
+//   [.., +4 C)           ctr[C]     as above
 // with Ei = kNoAllocMaxEdges, D = kNoAllocMaxDirFloats, C = kEdgeCtrInts.  Every call on a
 // device shares the array, so calls that overlap on the device race.
 // ---------------------------------------------------------------------------------

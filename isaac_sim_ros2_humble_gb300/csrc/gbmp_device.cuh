@@ -1,7 +1,8 @@
-// gbmp_device.cuh -- device-side data layout and the warp-per-state FK + collision
-// routine shared by every kernel of libgbmp.
+// gbmp_device.cuh -- device-side data layout, table staging, the lookup of a scene's distance
+// field, and the routines of one state a warp (FK, verdicts, costs).  Several states a warp:
+// gbmp_chunk_device.cuh (consecutive states of an edge), gbmp_states_device.cuh (any states).
 //
-// Execution model: one warp validates one joint state.
+// One state a warp:
 //   * FK: lanes 0..11 each own one element of the 3x4 pose of the current link and
 //     walk the chain link by link (KernelGenerator.h:369-400); the poses stay in the
 //     warp's shared-memory scratch, never in HBM unless the caller asks for them.

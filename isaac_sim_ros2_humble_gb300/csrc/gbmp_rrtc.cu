@@ -9,8 +9,8 @@
 //   2. draws a Philox sample in the joint limits (counter = lane, iteration),
 //   3. finds the nearest node of that tree (block-wide argmin over the active joints),
 //   4. steers to at most `range` (pRRTC.cu:415-434),
-//   5. validates the edge with the checkMotions step rule, one warp per state
-//      (FK + self + environment collision, broad phase included),
+//   5. validates the edge with the checkMotions step rule, by chunks of states where their
+//      scratch fits, else one warp per state (FK + self + environment collision),
 //   6. appends the node (atomic slot, NaN sentinel until every coordinate is written,
 //      pRRTC.cu:447-476 with the sentinel filled correctly),
 //   7. tries to connect: finds the nearest node of the other tree and extends towards
