@@ -4,6 +4,7 @@
 #pragma once
 
 #include <climits>
+#include <mutex>
 
 #include "gbmp_philox.h"
 #include "gbmp_rrtc.cuh"
@@ -495,9 +496,12 @@ __global__ void __launch_bounds__(kRrtcThreads, 4) k_rrtc_batch(const BatchProbl
 }
 
 
-// Raises a kernel's dynamic shared-memory limit to `smem`; never lowers it.
+// Raises a kernel's dynamic shared-memory limit to `smem`; never lowers it, also where several
+// threads launch it.
+inline std::mutex rrtc_limit_mutex;
 template <typename K>
 inline cudaError_t rrtc_raise_smem(K kern, size_t smem) {
+    std::lock_guard<std::mutex> lock(rrtc_limit_mutex);
     cudaFuncAttributes fa;
     const cudaError_t ce = cudaFuncGetAttributes(&fa, kern);
     if (ce != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return ce;
