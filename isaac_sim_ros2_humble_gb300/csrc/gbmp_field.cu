@@ -164,11 +164,14 @@ __global__ void __launch_bounds__(kFieldThreads)
 // if there are none), and reach no farther from their centres' median than kFieldReach times
 // what kFieldCore of them do (up to 1.6 in the scenes of the benchmarks, whose obstacles are
 // in one place).  One sphere 20 m away among 336 obstacles in a 1.2 m cube made cells of 0.67 m
-// instead of 0.07, and 70,000 states of the 8-DOF arm took 1,356 us; 57 us now.  Queries
-// outside the region go by its border cells, whose distances are to all obstacles.  The box of
-// all obstacles bounds what lies outside.  False when a number is not finite: the scene then
-// has no field, and every test runs.
-constexpr double kFieldCore = 0.875, kFieldReach = 2.0;
+// instead of 0.07, and 70,000 states of the 8-DOF arm took 1,356 us; 57 us now.  But more than
+// kFieldFew of the obstacles may be those around the robot: they stay in the grid unless its
+// cells then exceed kFieldCoarse metres (34 obstacles by the robot and 316 in a pile 5 m away,
+// cells of 0.2 m: 59 us, 122 with the grid over the pile alone; 30 m away 124 us with it).
+// Queries outside the region go by its border cells, whose distances are to all obstacles.  The
+// box of all obstacles bounds what lies outside.  False when a number is not finite: the scene
+// then has no field, and every test runs.
+constexpr double kFieldCore = 0.875, kFieldReach = 2.0, kFieldFew = 1.0 / 32, kFieldCoarse = 0.4;
 constexpr size_t kFieldSample = 256;
 bool scene_field_plan(const std::vector<double> &b, DevEnv &E, bool *tight) {
     const size_t n = b.size() / 4;
@@ -201,21 +204,35 @@ bool scene_field_plan(const std::vector<double> &b, DevEnv &E, bool *tight) {
     for (size_t k = 0; k < some; ++k) v[k] = reach[sample(k)];
     const size_t core = (size_t)std::ceil(kFieldCore * (double)some) - 1;
     std::nth_element(v.begin(), v.begin() + core, v.end());
-    const double farthest = kFieldReach * std::max(v[core], 0.0);
-    double slo[3] = {1e300, 1e300, 1e300}, shi[3] = {-1e300, -1e300, -1e300}, side = 0.0;
-    size_t outside = n - span.size();
-    for (double r : reach) outside += r > farthest;
-    for (int a = 0; a < 3; ++a) {
-        for (size_t k = 0; k < span.size(); ++k)
-            if (reach[k] <= farthest) {
-                slo[a] = std::min(slo[a], b[4 * span[k] + a] - b[4 * span[k] + 3]);
-                shi[a] = std::max(shi[a], b[4 * span[k] + a] + b[4 * span[k] + 3]);
-            }
-        slo[a] -= kFieldBorder;
-        shi[a] += kFieldBorder;
-        if (!(std::max(-slo[a], shi[a]) <= 2e6)) return false;
-        side = std::max(side, shi[a] - slo[a]);
+    double farthest = kFieldReach * std::max(v[core], 0.0);
+    double slo[3], shi[3], side;
+    auto box = [&] {   // of the spanning obstacles within `farthest`
+        side = 0.0;
+        for (int a = 0; a < 3; ++a) {
+            slo[a] = 1e300;
+            shi[a] = -1e300;
+            for (size_t k = 0; k < all; ++k)
+                if (reach[k] <= farthest) {
+                    slo[a] = std::min(slo[a], b[4 * span[k] + a] - b[4 * span[k] + 3]);
+                    shi[a] = std::max(shi[a], b[4 * span[k] + a] + b[4 * span[k] + 3]);
+                }
+            slo[a] -= kFieldBorder;
+            shi[a] += kFieldBorder;
+            side = std::max(side, shi[a] - slo[a]);
+        }
+    };
+    size_t beyond = 0;
+    for (double r : reach) beyond += r > farthest;
+    if ((double)beyond > kFieldFew * (double)all) {   // many: only where they would make the cells coarse
+        const double within = farthest;
+        farthest = 1e300;
+        box();
+        if (side > kFieldCoarse * kFieldCells) farthest = within;
+        else beyond = 0;
     }
+    box();
+    for (int a = 0; a < 3; ++a)
+        if (!(std::max(-slo[a], shi[a]) <= 2e6)) return false;
     if (!(side > 0.0)) return false;   // radii below 0
     const double h = side / kFieldCells;
     int cells[3];
@@ -224,7 +241,7 @@ bool scene_field_plan(const std::vector<double> &b, DevEnv &E, bool *tight) {
     E.ox = (float)slo[0]; E.oy = (float)slo[1]; E.oz = (float)slo[2];
     E.h = (float)h;
     E.inv_h = (float)(1.0 / h);
-    *tight = h <= kFieldFine && outside == 0;
+    *tight = h <= kFieldFine && beyond == 0 && all == n;
     for (int a = 0; a < 3; ++a) {   // outwards by more than single precision loses
         const double pad = 1e-5 + 1e-6 * std::max(std::fabs(lo[a]), std::fabs(hi[a]));
         (a == 0 ? E.lox : a == 1 ? E.loy : E.loz) = (float)(lo[a] - pad);

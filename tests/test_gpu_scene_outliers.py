@@ -42,6 +42,10 @@ def _scene(which):
     if which == "two places":     # three obstacles in four here, one in four 8 m away
         far = np.arange(256) % 4 == 0
         return dataclasses.replace(e, sphere_pos=e.sphere_pos + f(8) * far[:, None].astype(f))
+    if which in ("a pile 4 m away", "a pile 30 m away"):   # one obstacle in ten by the robot
+        here = np.arange(256) % 10 == 0
+        far = f(float(which.split()[2])) * (~here)[:, None].astype(f) * f([1, 0, 0])
+        return dataclasses.replace(e, sphere_pos=e.sphere_pos + far).subset(256, 0, 0)
     return e if which == "one place" else _sphere(e, {"20 m": (20, 20, 0), "1e4 m": (1e4, 0, 0), "1e9 m": (1e9, 0, 0),
                                                      "1e25 m": (0, -1e25, 0), "infinity": (-np.inf, 0, 0),
                                                      "no number": (np.nan, 0, 0)}[which])
@@ -57,7 +61,8 @@ def _check(R, E, q, cb=False):
     return v.cpu().numpy()
 
 
-@pytest.mark.parametrize("which", ["one place", "a floor", "a room", "two places", "20 m", "1e4 m", "1e9 m", "1e25 m",
+@pytest.mark.parametrize("which", ["one place", "a floor", "a room", "two places",
+                                   "a pile 4 m away", "a pile 30 m away", "20 m", "1e4 m", "1e9 m", "1e25 m",
                                    "infinity", "no number"])
 def test_verdicts_and_work(which):
     robot = W.serial_arm(2, dof=8, n_spheres=110, prismatic_torso=True)
